@@ -264,3 +264,72 @@ def tolerance(case):
     if case["dtype"] == "fp16":
         return {"rel": rel / 8, "max": most / 8}
     return {"rel": rel, "max": most}
+
+
+def _mm64(a, b):
+    """a @ b.T in 64 bits, a block of b's rows at a time."""
+    a = a.double()
+    out = torch.empty((a.shape[0], b.shape[0]), dtype=torch.float64, device=a.device)
+    for r in range(0, b.shape[0], 4096):
+        out[:, r:r + 4096] = a @ b[r:r + 4096].double().t()
+    return out
+
+
+def _grouped64(rows, weights, splits):
+    """Consecutive runs of `rows`, one per expert, each times its expert's weight."""
+    return torch.cat([_mm64(part, weights[e]) for e, part in enumerate(torch.split(rows, splits))])
+
+
+def _layer64(st):
+    """A MoE layer from its definition: rows sorted by expert (ties in token order), weighted sum over the choices."""
+    layer, x = st["layer"], st["x"]
+    logits = x.double() @ layer.router.double().t()
+    chosen = torch.topk(x.float() @ layer.router.t(), layer.topk, dim=1).indices  # which experts: a whole number
+    w = torch.softmax(logits.gather(1, chosen), dim=1).reshape(-1)
+    order = torch.argsort(chosen.reshape(-1), stable=True)
+    splits = torch.bincount(chosen.reshape(-1), minlength=layer.nexperts).tolist()
+    rows = x.double()[order // layer.topk]
+    h = _grouped64(rows, layer.w_up, splits)
+    if layer.w_gate is None:
+        h = torch.nn.functional.gelu(h)
+    else:
+        h = torch.nn.functional.silu(_grouped64(rows, layer.w_gate, splits)) * h
+    y = _grouped64(h, layer.w_down, splits) * w[order][:, None]
+    return torch.zeros_like(x, dtype=torch.float64).index_add_(0, order // layer.topk, y)
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "route":
+        return None
+    with torch.no_grad():
+        st = prepare(case, seed)
+        if kind in ("gemm", "ag"):
+            out = _mm64(st["a"], st["b"].t() if case.get("weight_kn") else st["b"])
+            if st["sa"] is not None:
+                out *= st["sa"].double()[:, None] * st["sb"].double()[None, :]
+            return out if st.get("bias") is None else out.add_(st["bias"])
+        if kind == "mlp":
+            y = _mm64(st["x"], st["w0"])
+            y = y if st["b0"] is None else y.add_(st["b0"])
+            z = _mm64(y, st["w1"])
+            return y, (z if st["b1"] is None else z.add_(st["b1"]))
+        if kind == "moe":
+            splits = st["splits_cpu"].tolist()
+            row_expert = torch.repeat_interleave(torch.arange(len(splits), device="cuda"), st["splits"].long())
+            source = torch.empty(row_expert.numel(), dtype=torch.int64, device="cuda")
+            source[st["si"].reshape(-1).long()] = torch.arange(source.numel(), device="cuda") // case["topk"]
+            y = _grouped64(st["x"].double()[source], st["w0"], splits)
+            if st["scale0"] is not None:
+                y *= st["scale0"].double()[row_expert][:, None]
+            z = _grouped64(y if st["act"] is None else st["act"], st["w1"], splits) * st["vec"].double()[:, None]
+            if st["scale1"] is not None:
+                z *= (st["in_scale"].double() * st["scale1"].double()[row_expert])[:, None]
+            return y, torch.zeros((case["tokens"], z.shape[1]), dtype=torch.float64, device="cuda").index_add_(0, source, z)
+        if kind == "layer":
+            return _layer64(st)
+    x = st["x"].detach().double().requires_grad_(True)
+    params = [p.detach().double().requires_grad_(True) for p in st["mlp"].parameters()]
+    w1, b1, w2, b2 = params if case["bias"] else (params[0], None, params[1], None)
+    y = torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(x, w1, b1)), w2, b2)
+    return (y.detach(),) + torch.autograd.grad(y, [x] + params, st["dy"].double())
