@@ -630,10 +630,20 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     if (lane == 0 && *s_abort != 0) drain_loads(stage, phase);
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA
-    if (lane == 0) {
+    // One thread issues all copies. It is picked with elect.sync, not by its lane number: only then does the
+    // compiler know that a single thread is active, and the copies' operands (which the hardware takes from
+    // registers shared by the warp) need no loop over the active lanes. The same holds for the UMMA thread below.
+    // Issuing one K block's two copies cost 330-370 clocks, its four UMMAs 380-460, behind `lane == 0`, more than
+    // the 512 a 256 x 256 tile's UMMAs take once the waits are added: every shape ran at 300 ns per K block.
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      // Pair mode: both CTAs' copies are credited to the leader's barrier, which the leader arms for the
+      // bytes of both.
+      const uint32_t full0 = CTA2 ? mapa_u32(bar_full(0), 0) : bar_full(0);
+      const bool arms = !CTA2 || leader;
+      const bool b_kn = p.b_mn_major != 0;
       int t, kb0, kb1, part;
       for (int wi = 0; ok && get_item(wi, t, kb0, kb1, part); ++wi) {
         TileCoord tc;
@@ -691,6 +701,11 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
             if (lead * kb_per_group > kb0) next_group_kb = lead >= ngroups ? 0x7fffffff : lead * kb_per_group;
           }
         }
+        // tiles of this rank's own shard read the caller's tensor in place
+        const bool own_a = p.a_own_valid && p.g_tiles == nullptr && tc.seg == p.rank;
+        const void* ta = own_a ? &p.tmap_a_own : &p.tmap_a;
+        const int arow = own_a ? tc.row0 - p.rank * p.seg_rows : tc.row0;
+        const int brow = tc.b_row0 + (CTA2 ? half * (BN / 2) : 0);  // first row (column of a [K, N] weight) of this CTA's share of B
         for (int kb = kb0; kb < kb1; ++kb) {
           if (kb == next_group_kb) {
             // entering a new slice group of the rows: wait (bounded) until all of its push units are in
@@ -707,51 +722,22 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
             ok = false;
             break;
           }
-          // Pair mode: both CTAs' copies are credited to the leader's barrier, which the leader
-          // arms for the bytes of both.
-          uint32_t fb = bar_full(stage);
-          if (CTA2) {
-            if (leader) mbar_arrive_expect_tx(fb, 2 * L::kStageBytes);
-            fb = mapa_u32(fb, 0);
-          } else {
-            mbar_arrive_expect_tx(fb, L::kStageBytes);
-          }
-          if (p.g_gather == nullptr) {
-            // tiles of this rank's own shard read the caller's tensor in place
-            const bool own_a = p.a_own_valid && p.g_tiles == nullptr && tc.seg == p.rank;
-            const void* ta = own_a ? &p.tmap_a_own : &p.tmap_a;
-            const int arow = own_a ? tc.row0 - p.rank * p.seg_rows : tc.row0;
-            if (CTA2) tma_load_2d_2cta(smem_a(stage), ta, fb, kb * BKE, arow);
-            else tma_load_2d(smem_a(stage), ta, fb, kb * BKE, arow);
-          } else {
-            // 32 gather4 copies of 4 rows each; rows past the tile end re-read a valid row
-            const int* gi = p.g_gather + (tc.rows > 0 ? tc.row0 : 0);
-            const int nr = tc.rows > 0 ? tc.rows : 1;
-            for (int q = 0; q < kBM / 4; ++q) {
-              const int r0 = q * 4;
-              const int i0 = gi[r0 < nr ? r0 : 0];
-              const int i1 = gi[r0 + 1 < nr ? r0 + 1 : 0];
-              const int i2 = gi[r0 + 2 < nr ? r0 + 2 : 0];
-              const int i3 = gi[r0 + 3 < nr ? r0 + 3 : 0];
-              if (CTA2)
-                tma_gather4_2d_2cta(smem_a(stage) + q * 4 * kRowBytes, &p.tmap_a, fb, kb * BKE, i0, i1, i2, i3);
-              else
-                tma_gather4_2d(smem_a(stage) + q * 4 * kRowBytes, &p.tmap_a, fb, kb * BKE, i0, i1, i2, i3);
-            }
-          }
-          if (p.b_mn_major) {
+          if (arms) mbar_arrive_expect_tx(bar_full(stage), CTA2 ? 2 * L::kStageBytes : L::kStageBytes);
+          const uint32_t fb = full0 + 8u * stage;
+          if (CTA2) tma_load_2d_2cta(smem_a(stage), ta, fb, kb * BKE, arow);
+          else tma_load_2d(smem_a(stage), ta, fb, kb * BKE, arow);
+          if (b_kn) {
             // B is [K, N]: one box of 64 columns x BKE rows per 64 output columns
             constexpr int kBoxes = L::kBRows / 64;
-            const int ncol0 = tc.b_row0 + (CTA2 ? half * (BN / 2) : 0);
 #pragma unroll
             for (int j = 0; j < kBoxes; ++j) {
-              if (CTA2) tma_load_2d_2cta(smem_b(stage) + j * (BKE * kRowBytes), &p.tmap_b, fb, ncol0 + j * 64, kb * BKE);
-              else tma_load_2d(smem_b(stage) + j * (BKE * kRowBytes), &p.tmap_b, fb, ncol0 + j * 64, kb * BKE);
+              if (CTA2) tma_load_2d_2cta(smem_b(stage) + j * (BKE * kRowBytes), &p.tmap_b, fb, brow + j * 64, kb * BKE);
+              else tma_load_2d(smem_b(stage) + j * (BKE * kRowBytes), &p.tmap_b, fb, brow + j * 64, kb * BKE);
             }
           } else if (CTA2) {
-            tma_load_2d_2cta(smem_b(stage), &p.tmap_b, fb, kb * BKE, tc.b_row0 + half * (BN / 2));
+            tma_load_2d_2cta(smem_b(stage), &p.tmap_b, fb, kb * BKE, brow);
           } else {
-            tma_load_2d(smem_b(stage), &p.tmap_b, fb, kb * BKE, tc.b_row0);
+            tma_load_2d(smem_b(stage), &p.tmap_b, fb, kb * BKE, brow);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -763,7 +749,15 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     }
   } else if (warp == 1) {
     // ----------------------------------------------------------------- UMMA
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {  // see the note on elect.sync above
+      const bool b_kn = p.b_mn_major != 0;
+      const bool acc_int = KIND == 1 && p.acc_int;
+      // Operand descriptors of stage 0; a later stage only moves the start address (bits [0,14), in units of 16 B).
+      // Each UMMA consumes 32 bytes of K of a K-major operand: advance the start address by 32 B
+      // (>>4 = 2); of an MN-major operand it consumes 16 K rows of 128 B: 2048 B (>>4 = 128)
+      const uint64_t a_desc0 = make_kmajor_sw128_desc(smem_a(0));
+      const uint64_t b_desc0 = b_kn ? make_mnmajor_sw128_desc(smem_b(0), BKE * kRowBytes) : make_kmajor_sw128_desc(smem_b(0));
+      const uint32_t b_step = b_kn ? 128u : 2u;
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -783,22 +777,19 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
           }
           tc_fence_after();
           if (tr != nullptr && it == 0 && kb == kb0) tr[1] = globaltimer_ns();
-          const uint64_t a_desc = make_kmajor_sw128_desc(smem_a(stage));
-          const uint64_t b_desc = p.b_mn_major ? make_mnmajor_sw128_desc(smem_b(stage), BKE * kRowBytes)
-                                               : make_kmajor_sw128_desc(smem_b(stage));
-          // each UMMA consumes 32 bytes of K of a K-major operand: advance the start address by 32 B
-          // (>>4 = 2); of an MN-major operand it consumes 16 K rows of 128 B: 2048 B (>>4 = 128)
-          const uint32_t b_step = p.b_mn_major ? 128u : 2u;
+          const uint32_t stage_off = static_cast<uint32_t>(stage) * (L::kStageBytes >> 4);
+          const uint64_t a_desc = a_desc0 + stage_off;
+          const uint64_t b_desc = b_desc0 + stage_off;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
             if (CTA2) {
               if (KIND == 0) umma_f16_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
-              else if (p.acc_int) umma_i8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
+              else if (acc_int) umma_i8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
               else umma_f8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
             } else {
               if (KIND == 0) umma_f16(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
-              else if (p.acc_int) umma_i8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
+              else if (acc_int) umma_i8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
               else umma_f8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
             }
           }
