@@ -256,6 +256,20 @@ inline void make_bands(GemmParams& p, int nseg, int tps, bool first_single, bool
   p.n_bands = nb;
 }
 
+// Split-K tail: into how many parts along K each of the `tail_tiles` tiles of the last, partial wave of `workers`
+// workers is cut (1 = not at all). A part of fewer than 8 K blocks, or a cut that saves fewer than 32, costs more than
+// it gives: the parts exchange their accumulators in about 10 us, a K block takes 0.17 (narrow tiles) to 0.28 us.
+// Measured, uncut / cut: 256 x 512 x 512 12.6 / 15.6 us; 256 x 2048 x 8192 54 / 29 us; 1 x 3584 x 8192 47 / 34 us.
+// A reduce-scatter launch (`scatter`) keeps four K blocks per part and no minimum: its whole tiles end with peers'
+// partials to fetch, work that a cut spreads as well, and it has only been timed on several GPUs that way.
+__host__ __device__ __forceinline__ int splitk_parts(int tail_tiles, int workers, int num_kb, bool scatter) {
+  if (tail_tiles <= 0 || 2 * tail_tiles > workers) return 1;
+  const int by_workers = workers / tail_tiles, by_k = num_kb / (scatter ? 4 : 8);
+  const int sp = by_workers < 8 ? by_workers : 8;
+  const int parts = sp < by_k ? sp : by_k;
+  return parts >= 2 && (scatter || num_kb - num_kb / parts >= 32) ? parts : 1;
+}
+
 // Split-K tail: which part finishes the 32-column step `c` of a tail tile that is BN columns wide and cut into
 // `split` parts. Steps are owned in pairs (one 64-column box = one staged store), box b by part
 // b * owners / boxes with owners = min(split, boxes); parts >= owners only park. A tile that is pushed to
@@ -353,6 +367,31 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 __device__ __forceinline__ uint32_t pack_f16(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Adds `parts` parked partial accumulators of a 32-column step, `stride` floats apart, to this part's: two parts' loads
+// in flight at a time. A part's step is 8 x 32 16-byte pieces, piece q of lane l at q * 32 + l (`src` is lane l's first).
+__device__ __forceinline__ void add_parked(uint32_t (&r)[32], const float* src, int stride, int parts, bool acc_int) {
+#pragma unroll 1
+  for (int sp = 0; sp < parts; sp += 2) {
+    const bool two = sp + 1 < parts;
+    uint4 pa[8], pb[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) pa[q] = *reinterpret_cast<const uint4*>(src + q * (32 * 4));
+#pragma unroll
+    for (int q = 0; q < 8; ++q) pb[q] = two ? *reinterpret_cast<const uint4*>(src + stride + q * (32 * 4)) : make_uint4(0u, 0u, 0u, 0u);
+    src += 2 * stride;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t wa[4] = {pa[q].x, pa[q].y, pa[q].z, pa[q].w}, wb[4] = {pb[q].x, pb[q].y, pb[q].z, pb[q].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t& x = r[q * 4 + j];
+        if (acc_int) x += wa[j] + wb[j];
+        else x = __float_as_uint((__uint_as_float(x) + __uint_as_float(wa[j])) + __uint_as_float(wb[j]));
+      }
+    }
+  }
 }
 
 // KIND: 0 = 16-bit inputs (bf16/f16 chosen by the instruction descriptor), 1 = fp8
@@ -456,13 +495,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
   const int full_waves = total_tiles / tile_step;
   const int full_tiles = full_waves * tile_step;
   const int tail_tiles = total_tiles - full_tiles;
-  int split = 1;
-  if (p.splitk_scratch != nullptr && p.g_tiles == nullptr && tail_tiles > 0 && 2 * tail_tiles <= tile_step) {
-    int sp = tile_step / tail_tiles;
-    if (sp > 8) sp = 8;
-    if (sp > num_kb / 4) sp = num_kb / 4;
-    if (sp >= 2) split = sp;
-  }
+  const int split = p.splitk_scratch != nullptr && p.g_tiles == nullptr ? splitk_parts(tail_tiles, tile_step, num_kb, p.epi_mode == kEpiRsPush) : 1;
   auto get_item = [&](int i, int& t, int& kb0, int& kb1, int& part) -> bool {
     part = 0;
     kb0 = 0;
@@ -832,16 +865,20 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       const uint32_t acc_phase = (it >> 1) & 1;
       TileCoord tc;
       decode_tile<BN, TILE_M>(p, t, m_tiles, n_tiles, tps, half, tc);
-      if (!mbar_wait(bar_tfull(acc), acc_phase, ab, kStatusTimeoutTmemFull, budget, 300)) break;
+      // (one verdict for the whole warp: what follows are warp-wide operations)
+      if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull(acc), acc_phase, ab, kStatusTimeoutTmemFull, budget, 300))) break;
       tc_fence_after();
-      // split-K tail: where this warp's 32 rows of a tail tile's partial accumulators live
+      // split-K tail: where this warp's 32 rows of a tail tile's partial accumulators live. Inside a part's slot the
+      // four columns q of 32-column step c of lane l are 16-byte piece (c * 8 + q) * 32 + l, so that every access of
+      // the warp is 512 contiguous bytes (stored row by row, 16 bytes per lane a kilobyte apart, the split tail of
+      // 2048 x 14336 x 4096 took 27 us).
       const bool is_tail = split > 1 && it == full_waves;
-      float* sk_rows = nullptr;
+      float* sk_warp = nullptr;
       int* sk_cnt = nullptr;
       int* sk_done = nullptr;
       if (is_tail) {
         const int tt = t - full_tiles;
-        sk_rows = p.splitk_scratch + (static_cast<long long>(tt) * (split - 1) * TILE_M + half * kBM + quad * 32 + lane) * BN;
+        sk_warp = p.splitk_scratch + (static_cast<long long>(tt) * (split - 1) * TILE_M + half * kBM + quad * 32) * BN + lane * 4;
         sk_cnt = p.splitk_cnt + (tt * 2 + half) * 4 + quad;
         sk_done = p.splitk_done + (tt * 2 + half) * 4 + quad;
       }
@@ -860,13 +897,13 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         for (int c = 0; c < BN / 32; ++c) {
           const int oc = sk_owner_of(c);
           if (oc == part) continue;
-          float* dst = sk_rows + static_cast<long long>(part < oc ? part : part - 1) * TILE_M * BN;
+          float* dst = sk_warp + static_cast<long long>(part < oc ? part : part - 1) * TILE_M * BN + c * (8 * 32 * 4);
           uint32_t r[32];
           tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * BN + c * 32), r);
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            *reinterpret_cast<uint4*>(dst + c * 32 + q * 4) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+            *reinterpret_cast<uint4*>(dst + q * (32 * 4)) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
         }
         __threadfence();
         __syncwarp();
@@ -959,10 +996,133 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
           bias_row = static_cast<const uint8_t*>(p.bias);
       }
 
-      // Plain output whose 32 rows of this warp are all valid: staged in shared memory and written with tiled
-      // stores (full 128-byte rows, one instruction per 32 x 64 box) instead of 16 bytes per lane per row.
-      const bool tma_out = p.tmap_out_valid && p.epi_mode == kEpiStore && otype != kOutF32 &&
-                           p.g_scatter_rows == nullptr && quad * 32 + 32 <= tc.rows;
+      // 16-bit output of the plain and grouped GEMMs with 16-byte aligned vectors, two 32-column steps (one 64-column
+      // box) per round. Rows leave through shared memory and tiled stores (full 128-byte rows, one instruction per
+      // 32 x 64 box) if all 32 rows of this warp are the tile's, or if nothing but the end of the output follows them
+      // (one segment: the map clips the rest); otherwise each lane stores its row's 16-byte pieces.
+      // Scales and bias are fetched 16 bytes at a time while the accumulator is read. The general loop below takes
+      // a branch per option and column and one dependent 2-byte load per bias element.
+      // 256 columns of a cold tile: 8500 clocks there (39000 with a row bias), 4900 (8500) here.
+      const bool tma_out = p.tmap_out_valid && p.epi_mode == kEpiStore && otype != kOutF32 && p.g_scatter_rows == nullptr &&
+                           (quad * 32 + 32 <= tc.rows || (p.g_tiles == nullptr && p.nseg == 1 && quad * 32 < tc.rows));
+      const bool lean = p.epi_mode == kEpiStore && otype != kOutF32 && (p.N & 7) == 0 && (p.ldo & 7) == 0 &&
+                        (p.scale_b == nullptr || (reinterpret_cast<uintptr_t>(p.scale_b) & 15) == 0) &&
+                        (p.bias_mode == kBiasNone || ((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0 && (p.ldbias & 7) == 0)) &&
+                        (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+      if (lean) {
+        const bool acc_int = KIND == 1 && p.acc_int;
+        const bool to_bf16 = otype == kOutBf16;
+        const float* sb_ptr = p.scale_b;
+        const bool has_bias = p.bias_mode != kBiasNone;
+        const bool bias_ok = p.bias_mode == kBiasRow || (p.bias_mode == kBiasFull && row_ok);
+#pragma unroll 1
+        for (int box = 0; box < BN / 64; ++box) {
+          const int box_col = tc.n0 + box * 64;
+          if (box_col >= p.N || quad * 32 >= tc.rows) break;
+          if (is_tail && sk_owner_of(2 * box) != part) continue;  // another part finishes this box
+          const uint32_t stage_blk = stage_blk0 + (L::kEpiBufs == 2 ? (box & 1) * L::kEpiBlockBytes : 0);
+          const uint32_t stage_row = stage_blk + lane * L::kEpiPitch;
+          if (tma_out) {
+            if (elect_one()) {  // the previous store out of this block has been read
+              if (L::kEpiBufs == 2) bulk_wait_read_keep1(); else bulk_wait_read();
+            }
+            __syncwarp();
+          }
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            const int c = 2 * box + h;
+            const int col0 = box_col + h * 32;
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * BN + c * 32), r);
+            tmem_ld_wait();
+            if (is_tail) add_parked(r, sk_warp + c * (8 * 32 * 4), TILE_M * BN, split - 1, acc_int);
+            float4 sb[8];
+            uint4 bv[4];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) sb[q] = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (sb_ptr != nullptr) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                if (col0 + q * 4 < p.N) sb[q] = __ldg(reinterpret_cast<const float4*>(sb_ptr + col0) + q);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bv[q] = make_uint4(0u, 0u, 0u, 0u);
+            if (bias_ok) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (col0 + q * 8 < p.N) bv[q] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(bias_row) + col0) + q);
+            }
+            if (acc_int) {
+              // int8 operands, int32 accumulator: dequantisation in the reference's order, bit-identical to its golden
+              // path (see the general loop); a bias joins the already rounded value
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float s4[4] = {sb[q].x, sb[q].y, sb[q].z, sb[q].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  float v = (row_scale * s4[j]) * __int2float_rn(static_cast<int>(r[q * 4 + j]));
+                  if (has_bias) v = to_bf16 ? __bfloat162float(__float2bfloat16_rn(v)) : __half2float(__float2half_rn(v));
+                  r[q * 4 + j] = __float_as_uint(v);
+                }
+              }
+            } else if (sb_ptr != nullptr) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float s4[4] = {sb[q].x, sb[q].y, sb[q].z, sb[q].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) r[q * 4 + j] = __float_as_uint((__uint_as_float(r[q * 4 + j]) * row_scale) * s4[j]);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * row_scale);
+            }
+            if (has_bias) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint32_t b4[4] = {bv[q].x, bv[q].y, bv[q].z, bv[q].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  float2 f;
+                  if (to_bf16) f = make_float2(__uint_as_float(b4[j] << 16), __uint_as_float(b4[j] & 0xFFFF0000u));
+                  else f = __half22float2(*reinterpret_cast<const __half2*>(&b4[j]));
+                  r[q * 8 + 2 * j] = __float_as_uint(__uint_as_float(r[q * 8 + 2 * j]) + f.x);
+                  r[q * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(r[q * 8 + 2 * j + 1]) + f.y);
+                }
+              }
+            }
+            uint32_t w[16];
+            if (to_bf16) {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) w[q] = pack_bf16(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1]));
+            } else {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) w[q] = pack_f16(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1]));
+            }
+            if (tma_out) {
+              // 128-byte rows, 16-byte pieces XOR-swizzled by row like the tensor map's 128-byte swizzle
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage_row + (((h * 4 + q) ^ (lane & 7)) << 4)),
+                             "r"(w[4 * q]), "r"(w[4 * q + 1]), "r"(w[4 * q + 2]), "r"(w[4 * q + 3])
+                             : "memory");
+            } else if (row_ok) {
+              uint16_t* d = reinterpret_cast<uint16_t*>(dst_row) + col0;
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (col0 + q * 8 < p.N)
+                  *reinterpret_cast<uint4*>(d + q * 8) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+            }
+          }
+          if (tma_out) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (elect_one()) {
+              tma_store_2d(&p.tmap_out, stage_blk, box_col, tc.row0 + quad * 32);
+              bulk_commit();
+            }
+          }
+        }
+      } else
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         if (is_tail && sk_owner_of(c) != part) continue;  // another part finishes this box
@@ -973,30 +1133,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         tmem_ld_wait();
         const int col0 = tc.n0 + c * 32;
         const bool active = row_ok && col0 < p.N;
-        if (is_tail) {
-          // add the parked partial accumulators of the other K parts, two parts' loads in flight at a time
-          for (int sp = 0; sp < split - 1; sp += 2) {
-            float4 pv[2][8];
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-              if (sp + u < split - 1) {
-                const float* src = sk_rows + static_cast<long long>(sp + u) * TILE_M * BN + c * 32;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) pv[u][q] = *reinterpret_cast<const float4*>(src + q * 4);
-              }
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-              if (sp + u < split - 1) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  r[q * 4] = __float_as_uint(__uint_as_float(r[q * 4]) + pv[u][q].x);
-                  r[q * 4 + 1] = __float_as_uint(__uint_as_float(r[q * 4 + 1]) + pv[u][q].y);
-                  r[q * 4 + 2] = __float_as_uint(__uint_as_float(r[q * 4 + 2]) + pv[u][q].z);
-                  r[q * 4 + 3] = __float_as_uint(__uint_as_float(r[q * 4 + 3]) + pv[u][q].w);
-                }
-              }
-          }
-        }
+        if (is_tail) add_parked(r, sk_warp + c * (8 * 32 * 4), TILE_M * BN, split - 1, KIND == 1 && p.acc_int);
         float v[32];
         if (KIND == 1 && p.acc_int) {
           // int8 operands, int32 accumulator. Dequantisation in the reference's order, so that the result is
@@ -1132,36 +1269,6 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
               bulk_commit();
             }
           }
-        } else if (tma_out) {
-          // same staging as the 16-bit reduce-scatter push, into the output tensor itself
-          const int box = c >> 1, h = c & 1;
-          const uint32_t stage_blk = stage_blk0 + (L::kEpiBufs == 2 ? (box & 1) * L::kEpiBlockBytes : 0);
-          const uint32_t stage_row = stage_blk + lane * L::kEpiPitch;
-          if (h == 0) {
-            if (lane == 0) {  // the previous store out of this block has been read
-              if (L::kEpiBufs == 2) bulk_wait_read_keep1(); else bulk_wait_read();
-            }
-            __syncwarp();
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              w[j] = (otype == kOutBf16) ? pack_bf16(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1])
-                                         : pack_f16(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage_row + (((h * 4 + q) ^ (lane & 7)) << 4)),
-                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
-                         : "memory");
-          }
-          if (h == 1) {
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (col0 - 32 < p.N) tma_store_2d(&p.tmap_out, stage_blk, col0 - 32, tc.row0 + quad * 32);
-              bulk_commit();
-            }
-          }
         } else if (p.epi_mode == kEpiRsPush && !own) {
           // fp32 wire format. Park the warp's 32 x 32 fp32 block in shared memory (lane = row, 16-byte pieces XOR-swizzled
           // by row so that the writes spread over all banks and match the tensor map's 128-byte swizzle),
@@ -1222,6 +1329,10 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         __syncwarp();
       }
       tc_fence_before();
+      if (p.gr_slab_done != nullptr && tma_out && elect_one()) {  // MoE layer 1: the tile's stores are complete before they are announced
+        bulk_wait_all();
+        fence_proxy_async();
+      }
       __syncwarp();
       if (lane == 0) {
         if (CTA2) mbar_arrive_cluster(mapa_u32(bar_tempty(acc), 0));
@@ -1229,10 +1340,6 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         // MoE layer 1: this warp's rows of the tile are stored (tiled stores complete, and the release covers
         // the whole warp's plain stores)
         if (p.gr_slab_done != nullptr) {
-          if (tma_out) {
-            bulk_wait_all();
-            fence_proxy_async();
-          }
           red_add_release_gpu(p.gr_slab_done + tc.n_idx, 1);
         }
       }
@@ -1271,7 +1378,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       }
     }
     if (tr != nullptr && warp == 2 && lane == 0) tr[3] = globaltimer_ns();
-    if (p.epi_mode == kEpiStore && p.tmap_out_valid && lane == 0) bulk_wait_all();  // tiled stores must not outlive the CTA
+    if (p.epi_mode == kEpiStore && p.tmap_out_valid && elect_one()) bulk_wait_all();  // tiled stores must not outlive the CTA
     if (p.epi_mode == kEpiRsPush && lane == 0) {
       // also on the way out after a failed wait: the stores must not outlive the CTA
       bulk_wait_all();

@@ -215,7 +215,12 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
     const long long tiles = static_cast<long long>(p.nseg) * ((p.seg_rows + tile_m - 1) / tile_m) *
                             ((p.N + bn - 1) / bn) * (cg == 2 ? 2 : 1);
     // the all-gather push is spread over every CTA's comm warps, so keep the full grid there
-    if (p.ag_src == nullptr && tiles < grid) grid = static_cast<int>(tiles);
+    if (p.ag_src == nullptr && tiles < grid) {
+      // less than one wave: as many CTAs as the split-K schedule has work for
+      const int per = cg == 2 ? 2 : 1;
+      const int num_kb = static_cast<int>((static_cast<long long>(p.K) * dtype_bytes(in_dtype) + kRowBytes - 1) / kRowBytes);
+      grid = static_cast<int>(tiles) * splitk_parts(static_cast<int>(tiles) / per, grid / per, num_kb, p.epi_mode == kEpiRsPush);
+    }
   }
   if (grid < 1) grid = 1;
   if (p.group_m <= 0) p.group_m = (tuning != nullptr && tuning->group_m > 0) ? tuning->group_m : 8;
@@ -242,7 +247,6 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
   p.acc_int = is_int8(in_dtype) ? 1 : 0;
   if (p.acc_int) {
     FLUXB_REQUIRE(p.out_type != kOutF32 || p.epi_mode == kEpiRsPush, "int8 inputs produce a 16-bit output");
-    p.splitk_scratch = nullptr;  // the split-K tail adds parked accumulators as fp32: not for int32 accumulators
   }
   const uint32_t idesc = make_idesc(fmt, cg == 2 ? 2 * kBM : kBM, static_cast<uint32_t>(bn), p.b_mn_major ? 1u : 0u,
                                     p.acc_int ? 2u : 1u);

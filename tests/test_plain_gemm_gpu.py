@@ -1,0 +1,83 @@
+"""The plain GEMM's epilogue and split last wave at the sizes and options where they can go wrong: rows and columns
+that end inside a warp's 32 rows or a 64-column box, vectors that are not 16-byte aligned, K cut over several CTAs.
+
+Bound of every element: half a unit in the last place of the 16-bit output, taken twice (2^-8 of the value for bf16,
+2^-11 for fp16), plus K roundings of fp32 sums, K * 2^-23 * sum |a| |b|. int8 is compared bit for bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF16, FP16 = torch.bfloat16, torch.float16
+
+
+@pytest.fixture(scope="module")
+def flux():
+    import flux_b200
+
+    flux_b200.init_flux_shm(None)
+    flux_b200.get_comm(None).set_timeout_ms(5000)
+    return flux_b200
+
+
+def _inputs(m, n, k, dtype, seed=5):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    a = torch.randn(m, k, generator=g, device="cuda").to(dtype)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.02).to(dtype)
+    return a, b, g
+
+
+def _check(flux, out, a, b, extra=None):
+    torch.cuda.synchronize()
+    flux.get_comm(None).check_status()
+    ref = a.double() @ b.double().t()
+    if extra is not None:
+        ref = ref + extra.double()
+    bound = ref.abs() * (2.0 ** -8 if out.dtype == BF16 else 2.0 ** -11)
+    bound += a.shape[1] * 2.0 ** -23 * (a.double().abs() @ b.double().abs().t()) + 1e-6
+    worst = ((out.double() - ref).abs() / bound).max().item()
+    assert worst <= 1.0, f"{worst:.2f} times the bound"
+
+
+@pytest.mark.parametrize("dtype", [BF16, FP16])
+@pytest.mark.parametrize("m,n,k,tuning", [
+    (1, 8, 64, None), (31, 72, 128, None), (33, 56, 512, None), (289, 328, 320, {"cta_group": 2}), (300, 200, 192, {"cta_group": 1}),
+    (130, 264, 8192, {"block_n": 64, "cta_group": 1}), (257, 512, 4096, {"block_n": 256, "cta_group": 2}),
+])
+@pytest.mark.parametrize("bias", ["none", "row", "full", "row unaligned", "full unaligned"])
+def test_epilogue_edges(flux, m, n, k, tuning, bias, dtype):
+    a, b, g = _inputs(m, n, k, dtype)
+    rows = m if bias.startswith("full") else 1
+    t = None
+    if bias != "none":
+        flat = torch.randn(rows * n + 1, generator=g, device="cuda").to(dtype)
+        t = (flat[1:] if "unaligned" in bias else flat[:-1]).view(rows, n)
+    out = flux.GemmOnly(dtype).forward(a, b, bias=t, tuning=tuning)
+    _check(flux, out, a, b, t)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_column_scales_of_any_alignment(flux, shift):
+    m, n, k = 200, 264, 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    sa = torch.rand(m, generator=g, device="cuda") * 0.01 + 0.001
+    sb = (torch.rand(n + 1, generator=g, device="cuda") * 0.01 + 0.001)[shift:n + shift]
+    out = flux.GemmOnly(torch.int8).forward(a, b, input_scale=sa, weight_scale=sb)
+    torch.cuda.synchronize()
+    acc = (a.double() @ b.double().t()).float()  # exact: below 2^24
+    assert torch.equal(out, ((sa[:, None] * sb[None, :]) * acc).to(BF16))
+
+
+@pytest.mark.parametrize("m,n,tuning", [(130, 72, {"block_n": 64, "cta_group": 1}), (300, 520, {"block_n": 256, "cta_group": 2})])
+def test_int8_accumulators_cut_along_k_stay_whole_numbers(flux, m, n, tuning):
+    k = 8192  # 64 K blocks: cut into up to eight parts
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    ones_m, ones_n = torch.ones(m, device="cuda"), torch.ones(n, device="cuda")
+    for _ in range(2):  # the counters of the parts clear themselves
+        out = flux.GemmOnly(torch.int8).forward(a, b, input_scale=ones_m, weight_scale=ones_n, tuning=tuning)
+        torch.cuda.synchronize()
+        flux.get_comm(None).check_status()
+        assert torch.equal(out, (a.double() @ b.double().t()).float().to(BF16))
