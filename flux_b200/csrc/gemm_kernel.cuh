@@ -259,7 +259,8 @@ inline void make_bands(GemmParams& p, int nseg, int tps, bool first_single, bool
 // Split-K tail: into how many parts along K each of the `tail_tiles` tiles of the last, partial wave of `workers`
 // workers is cut (1 = not at all). A part of fewer than 8 K blocks, or a cut that saves fewer than 32, costs more than
 // it gives: the parts exchange their accumulators in about 10 us, a K block takes 0.17 (narrow tiles) to 0.28 us.
-// Measured, uncut / cut: 256 x 512 x 512 12.6 / 15.6 us; 256 x 2048 x 8192 54 / 29 us; 1 x 3584 x 8192 47 / 34 us.
+// Measured with a grid large enough to cut whole launches, uncut / cut: 256 x 512 x 512 12.6 / 15.6 us; 256 x 2048 x
+// 8192 54 / 29 us.
 // A reduce-scatter launch (`scatter`) keeps four K blocks per part and no minimum: its whole tiles end with peers'
 // partials to fetch, work that a cut spreads as well, and it has only been timed on several GPUs that way.
 __host__ __device__ __forceinline__ int splitk_parts(int tail_tiles, int workers, int num_kb, bool scatter) {
@@ -470,9 +471,14 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     }
   }
   tc_fence_before();
+  // A dense plain GEMM touches global memory first with its producer's loads, which wait there; every other mode reads
+  // tables, counters or tokens in several roles.
+  const bool pdl_late = p.g_tiles == nullptr && p.epi_mode == kEpiStore && p.ag_flags == nullptr && p.ag_src == nullptr;
+  if (!pdl_late) pdl_wait();
   if (CTA2) cluster_sync_all(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if (threadIdx.x == 0) pdl_trigger();
 
   const int n_tiles = (p.N + BN - 1) / BN;
   int tps = 1, m_tiles;
@@ -738,6 +744,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         const bool own_a = p.a_own_valid && p.g_tiles == nullptr && tc.seg == p.rank;
         const void* ta = own_a ? &p.tmap_a_own : &p.tmap_a;
         const int arow = own_a ? tc.row0 - p.rank * p.seg_rows : tc.row0;
+        if (wi == 0 && pdl_late) pdl_wait();
         const int brow = tc.b_row0 + (CTA2 ? half * (BN / 2) : 0);  // first row (column of a [K, N] weight) of this CTA's share of B
         for (int kb = kb0; kb < kb1; ++kb) {
           if (kb == next_group_kb) {

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "skinny_gemm.cuh"
 
 namespace fluxb {
 
@@ -14,6 +15,8 @@ namespace fluxb {
 // ---------------------------------------------------------------------------
 template <int BN, int STAGES, int KIND, bool CTA2>
 static int launch_inst(const fluxb_comm* comm, const GemmParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+  // (several ranks: the launch order of kernels that wait on one another stays the stream's)
+  const bool pdl = comm->world == 1;
   using L = SmemLayout<BN, STAGES, CTA2>;
   auto kern = fused_gemm_kernel<BN, STAGES, KIND, CTA2>;
   static bool configured[64] = {};
@@ -26,11 +29,13 @@ static int launch_inst(const fluxb_comm* comm, const GemmParams& p, uint32_t ide
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = L::kTotal;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CTA2 ? 2 : 1;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (!configured[dev]) {
@@ -51,6 +56,7 @@ static int launch_inst(const fluxb_comm* comm, const GemmParams& p, uint32_t ide
     if (grid < 2) grid = 2;
   }
   cfg.gridDim = dim3(grid, 1, 1);
+  if (pdl) cfg.numAttrs = 2;
   FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, idesc));
   return FLUXB_OK;
 }
@@ -200,6 +206,17 @@ int enqueue_or_defer(fluxb_comm* comm, cudaStream_t stream, std::function<int(cu
   return FLUXB_OK;
 }
 
+static int input_format(int in_dtype, uint32_t* fmt) {
+  switch (in_dtype) {
+    case FLUXB_BF16: *fmt = 1; return FLUXB_OK;
+    case FLUXB_F16: *fmt = 0; return FLUXB_OK;
+    case FLUXB_E4M3: *fmt = 0; return FLUXB_OK;
+    case FLUXB_E5M2: *fmt = 1; return FLUXB_OK;
+    case FLUXB_S8: *fmt = 1; return FLUXB_OK;
+    default: FLUXB_FAIL(FLUXB_ERR_INVALID, "input dtype %d is not bf16/f16/e4m3/e5m2/s8", in_dtype);
+  }
+}
+
 int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
                       const fluxb_tuning* tuning, cudaStream_t stream) {
   const int cg = resolve_cta_group(p, tuning);
@@ -215,12 +232,7 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
     const long long tiles = static_cast<long long>(p.nseg) * ((p.seg_rows + tile_m - 1) / tile_m) *
                             ((p.N + bn - 1) / bn) * (cg == 2 ? 2 : 1);
     // the all-gather push is spread over every CTA's comm warps, so keep the full grid there
-    if (p.ag_src == nullptr && tiles < grid) {
-      // less than one wave: as many CTAs as the split-K schedule has work for
-      const int per = cg == 2 ? 2 : 1;
-      const int num_kb = static_cast<int>((static_cast<long long>(p.K) * dtype_bytes(in_dtype) + kRowBytes - 1) / kRowBytes);
-      grid = static_cast<int>(tiles) * splitk_parts(static_cast<int>(tiles) / per, grid / per, num_kb, p.epi_mode == kEpiRsPush);
-    }
+    if (p.ag_src == nullptr && tiles < grid) grid = static_cast<int>(tiles);
   }
   if (grid < 1) grid = 1;
   if (p.group_m <= 0) p.group_m = (tuning != nullptr && tuning->group_m > 0) ? tuning->group_m : 8;
@@ -236,14 +248,8 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
   p.world = comm->world;
   const int kind = is_8bit(in_dtype) ? 1 : 0;
   uint32_t fmt;
-  switch (in_dtype) {
-    case FLUXB_BF16: fmt = 1; break;
-    case FLUXB_F16: fmt = 0; break;
-    case FLUXB_E4M3: fmt = 0; break;
-    case FLUXB_E5M2: fmt = 1; break;
-    case FLUXB_S8: fmt = 1; break;
-    default: FLUXB_FAIL(FLUXB_ERR_INVALID, "input dtype %d is not bf16/f16/e4m3/e5m2/s8", in_dtype);
-  }
+  const int rc_fmt = input_format(in_dtype, &fmt);
+  if (rc_fmt != FLUXB_OK) return rc_fmt;
   p.acc_int = is_int8(in_dtype) ? 1 : 0;
   if (p.acc_int) {
     FLUXB_REQUIRE(p.out_type != kOutF32 || p.epi_mode == kEpiRsPush, "int8 inputs produce a 16-bit output");
@@ -274,6 +280,120 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
     default: return FLUXB_LAUNCH(64, stages_for(64, false), stages_for(64, true));
   }
 #undef FLUXB_LAUNCH
+}
+
+// ---------------------------------------------------------------------------
+// few rows (skinny_gemm.cuh)
+// ---------------------------------------------------------------------------
+template <int BN, int KIND>
+static int launch_skinny_inst(const SkinnyParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+  auto kern = skinny_gemm_kernel<BN, KIND>;
+  static bool configured[64] = {};
+  int dev = 0;
+  FLUXB_CUDA(cudaGetDevice(&dev));
+  FLUXB_REQUIRE(dev < 64, "device index %d not supported", dev);
+  if (!configured[dev]) {
+    FLUXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SkinnyLayout<BN>::kTotal));
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(kSkinnyThreads, 1, 1);
+  cfg.dynamicSmemBytes = SkinnyLayout<BN>::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, idesc));
+  return FLUXB_OK;
+}
+
+// Token columns of a skinny launch's tile.
+static int skinny_block(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : m <= 128 ? 128 : 256; }
+
+// Into how many parts along K the tiles of a skinny launch are cut: as many as keep all CTAs resident (two per SM up
+// to 64 tokens; one above, where clusters of four leave a few SMs idle) with at least 4 K blocks each. Measured (us,
+// inputs in L2 where they fit; 1 / 2 / 4 / 8 parts): 1 x 3584 x 8192 22.7 / 14.5 / 10.4 / 10.4, 1 x 8192 x 3584 13.7 / 10.4 /
+// 11.0 / 14.5, 48 x 6144 x 12288 62 / 39 / 33 / 37, 48 x 12288 x 6144 39 / 33 / 37 / 41, 128 x 4096 x 4096 20 / 14.5 / 12.4 / 25.
+static int skinny_split(int sm_count, int n_tiles, int num_kb, int bn) {
+  const int slots = bn <= 64 ? 2 * sm_count : sm_count - sm_count / 8;
+  const int most = bn <= 64 ? kSkinnyMaxSplit : 4;
+  int split = 1;
+  while (split < most && 2 * split * n_tiles <= slots && num_kb / (2 * split) >= 4) split *= 2;
+  return split;
+}
+
+// Where the skinny kernel takes over from the fused one's tiles (us, fused / skinny): every shape up to 64 rows
+// (16 x 4096 x 4096 22.8 / 9.0); above, shapes whose weights are too narrow to fill the GPU, so that K is cut at
+// least twice up to 128 rows (128 x 4096 x 4096 22.9 / 10.5 in four parts, but 128 x 14336 x 4096 26.4 / 30.9 in
+// one) and four times up to 256 (256 x 2048 x 8192 54 / 22.6, but 256 x 8192 x 8192 36 / 42 in two): the partial sums of
+// that many tokens take longer to exchange.
+static bool skinny_wins(int sm_count, int m, int n, long long row_bytes) {
+  if (m > kSkinnyMaxM) return false;
+  if (m <= 64) return true;
+  const int num_kb = static_cast<int>((row_bytes + kRowBytes - 1) / kRowBytes);
+  return skinny_split(sm_count, (n + kBM - 1) / kBM, num_kb, skinny_block(m)) >= (m <= 128 ? 2 : 4);
+}
+
+// The plain GEMM of m <= kSkinnyMaxM rows with a 16-bit output and 4-byte aligned output and bias.
+static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, void* c, int m, int n, int k, int in_dtype,
+                         int out_type, const void* bias, int bias_mode, const float* scale_a, const float* scale_b,
+                         float alpha, int flags, cudaStream_t stream) {
+  SkinnyParams p;
+  memset(&p, 0, sizeof(p));
+  const int eb = dtype_bytes(in_dtype);
+  const int bn = skinny_block(m);
+  const long long row_bytes = static_cast<long long>(k) * eb;
+  p.M = m;
+  p.N = n;
+  p.num_kb = static_cast<int>((row_bytes + kRowBytes - 1) / kRowBytes);
+  p.w_kn = (flags & FLUXB_WEIGHT_KN) ? 1 : 0;
+  p.acc_int = is_int8(in_dtype) ? 1 : 0;
+  p.out_bf16 = out_type == kOutBf16 ? 1 : 0;
+  p.bias_mode = bias_mode;
+  p.out = static_cast<uint16_t*>(c);
+  p.bias = static_cast<const uint16_t*>(bias);
+  p.scale_a = scale_a;
+  p.scale_b = scale_b;
+  p.ldo = p.ldbias = n;
+  p.alpha = alpha;
+  p.timeout_ns = comm->timeout_ns;
+  p.status = comm->status_dev;
+  p.trace = comm->trace;
+  int rc;
+  if (p.w_kn) {
+    FLUXB_REQUIRE(is_16bit(in_dtype), "a [K,N] weight needs 16-bit inputs (fp8 forbids transpose_weight)");
+    rc = encode_tmap_kn(&p.tmap_w, b, in_dtype, k, n, static_cast<long long>(n) * eb, kRowBytes / eb);
+  } else {
+    rc = encode_tmap_2d(&p.tmap_w, b, in_dtype, n, k, row_bytes, kBM);
+  }
+  if (rc != FLUXB_OK) return rc;
+  rc = encode_tmap_2d(&p.tmap_x, a, in_dtype, m, k, row_bytes, bn);
+  if (rc != FLUXB_OK) return rc;
+  uint32_t fmt;
+  rc = input_format(in_dtype, &fmt);
+  if (rc != FLUXB_OK) return rc;
+  const uint32_t idesc = make_idesc(fmt, kBM, static_cast<uint32_t>(bn), 0u, p.acc_int ? 2u : 1u, p.w_kn ? 1u : 0u);
+  const int n_tiles = (n + kBM - 1) / kBM;
+  p.split = skinny_split(comm->sm_count, n_tiles, p.num_kb, bn);
+  const int grid = n_tiles * p.split;
+#define FLUXB_SKINNY(BN_) \
+  (is_8bit(in_dtype) ? launch_skinny_inst<BN_, 1>(p, idesc, grid, stream) : launch_skinny_inst<BN_, 0>(p, idesc, grid, stream))
+  switch (bn) {
+    case 16: return FLUXB_SKINNY(16);
+    case 32: return FLUXB_SKINNY(32);
+    case 64: return FLUXB_SKINNY(64);
+    case 128: return FLUXB_SKINNY(128);
+    default: return FLUXB_SKINNY(256);
+  }
+#undef FLUXB_SKINNY
 }
 
 static int out_type_of(int out_dtype, int* ot) {
@@ -367,6 +487,12 @@ int fluxb_gemm(fluxb_comm_t comm, const void* a, const void* b, void* c, int m, 
   const int eb = dtype_bytes(in_dtype);
   rc = out_type_of(out_dtype, &p.out_type);
   if (rc != FLUXB_OK) return rc;
+  // a caller who chose a tile shape or grid gets the fused kernel's
+  const bool chosen = tuning != nullptr && (tuning->block_n != 0 || tuning->cta_group != 0 || tuning->num_ctas != 0 || tuning->group_m != 0);
+  if (!chosen && skinny_wins(comm->sm_count, m, n, static_cast<long long>(k) * eb) && comm->ranks_on_gpu <= 1 && p.out_type != kOutF32 &&
+      ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(bias_mode != FLUXB_BIAS_NONE ? bias : nullptr)) & 3) == 0)
+    return launch_skinny(comm, a, b, c, m, n, k, in_dtype, p.out_type, bias, bias_mode, scale_a, scale_b, alpha, flags,
+                         static_cast<cudaStream_t>(stream));
   p.M = m;
   p.N = n;
   p.K = k;

@@ -41,7 +41,7 @@ def _check(flux, out, a, b, extra=None):
 @pytest.mark.parametrize("dtype", [BF16, FP16])
 @pytest.mark.parametrize("m,n,k,tuning", [
     (1, 8, 64, None), (31, 72, 128, None), (33, 56, 512, None), (289, 328, 320, {"cta_group": 2}), (300, 200, 192, {"cta_group": 1}),
-    (130, 264, 8192, {"block_n": 64, "cta_group": 1}), (257, 512, 4096, {"block_n": 256, "cta_group": 2}),
+    (130, 264, 512, {"block_n": 64, "cta_group": 1}), (257, 512, 1024, {"block_n": 256, "cta_group": 2}),
 ])
 @pytest.mark.parametrize("bias", ["none", "row", "full", "row unaligned", "full unaligned"])
 def test_epilogue_edges(flux, m, n, k, tuning, bias, dtype):
@@ -53,6 +53,50 @@ def test_epilogue_edges(flux, m, n, k, tuning, bias, dtype):
         t = (flat[1:] if "unaligned" in bias else flat[:-1]).view(rows, n)
     out = flux.GemmOnly(dtype).forward(a, b, bias=t, tuning=tuning)
     _check(flux, out, a, b, t)
+
+
+@pytest.mark.parametrize("kn", [False, True])
+@pytest.mark.parametrize("m", [1, 2, 16, 17, 32, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("n,k", [(8, 64), (136, 264), (1160, 4096), (5000, 1032)])  # cut along K into 1, 1, 8 or 4, 4 or 2 parts
+def test_few_rows(flux, m, n, k, kn):
+    a, b, g = _inputs(m, n, k, BF16, seed=m + n)
+    bias = torch.randn(m if m % 2 else 1, n, generator=g, device="cuda").to(BF16)
+    out = flux.GemmOnly(BF16, transpose_weight=kn).forward(a, b.t().contiguous() if kn else b, bias=bias)
+    _check(flux, out, a, b, bias)
+
+
+@pytest.mark.parametrize("m", [3, 40, 100, 200])
+def test_few_rows_8bit(flux, m):
+    n, k = 1288, 4112
+    g = torch.Generator(device="cuda").manual_seed(m)
+    sa, sb = torch.rand(m, generator=g, device="cuda") * 0.01 + 0.001, torch.rand(n, generator=g, device="cuda") * 0.01 + 0.001
+    ai = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    bi = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    bias = torch.randn(1, n, generator=g, device="cuda").to(BF16)
+    out = flux.GemmOnly(torch.int8).forward(ai, bi, bias=bias, input_scale=sa, weight_scale=sb)
+    torch.cuda.synchronize()
+    acc = (ai.double() @ bi.double().t()).float()
+    assert torch.equal(out, ((sa[:, None] * sb[None, :]) * acc).to(BF16) + bias)
+    a8, b8 = torch.randn(m, k, generator=g, device="cuda").to(torch.float8_e4m3fn), torch.randn(n, k, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    out = flux.GemmOnly(torch.float8_e4m3fn).forward(a8, b8, input_scale=sa, weight_scale=sb)
+    _check(flux, out, a8.double() * sa[:, None].double(), b8.double() * sb[:, None].double())
+
+
+def test_few_rows_on_two_streams(flux):
+    """Launches that run side by side share nothing: same result as one after the other."""
+    a, b, _ = _inputs(16, 2048, 4096, BF16)
+    a2 = a.flip(0).contiguous()
+    op = flux.GemmOnly(BF16)
+    want, want2 = op.forward(a, b), op.forward(a2, b)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = [[], []]
+    for _ in range(20):
+        for i, x in enumerate((a, a2)):
+            with torch.cuda.stream(streams[i]):
+                outs[i].append(op.forward(x, b))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs[0]) and all(torch.equal(o, want2) for o in outs[1])
 
 
 @pytest.mark.parametrize("shift", [0, 1])
@@ -69,9 +113,10 @@ def test_column_scales_of_any_alignment(flux, shift):
     assert torch.equal(out, ((sa[:, None] * sb[None, :]) * acc).to(BF16))
 
 
-@pytest.mark.parametrize("m,n,tuning", [(130, 72, {"block_n": 64, "cta_group": 1}), (300, 520, {"block_n": 256, "cta_group": 2})])
+@pytest.mark.parametrize("m,n,tuning", [(130, 72 + 64 * 4, {"block_n": 64, "cta_group": 1, "num_ctas": 8}),
+                                        (300, 1288, {"block_n": 256, "cta_group": 2, "num_ctas": 16})])
 def test_int8_accumulators_cut_along_k_stay_whole_numbers(flux, m, n, tuning):
-    k = 8192  # 64 K blocks: cut into up to eight parts
+    k = 8192  # 64 K blocks; 12 tiles on 8 workers: the last 4 (two) are cut into 2 (four) parts
     g = torch.Generator(device="cuda").manual_seed(4)
     a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
     b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
