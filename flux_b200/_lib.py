@@ -107,6 +107,7 @@ SIGNATURES = {
     "fluxb_moe_ag_scatter_destroy": (_i, [_vp]),
     "fluxb_moe_ag_scatter_reset": (_i, [_vp, _vp]),
     "fluxb_moe_ag_scatter_set_ep": (_i, [_vp, _i, _i]),
+    "fluxb_moe_ag_scatter_keep_tokens": (_i, [_vp, _i]),
     "fluxb_moe_ag_scatter_forward": (_i, [_vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _tun, _vp]),
     "fluxb_moe_scatter_gemm_static": (_i, [_vp, _vp, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _tun, _vp]),
     "fluxb_moe_gather_rs_workspace_bytes": (_sz, [_i, _i, _i, _i]),

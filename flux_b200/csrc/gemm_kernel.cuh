@@ -50,6 +50,7 @@ constexpr int kMaxWorld = 8;
 constexpr int kCommSliceBytes = 2048;  // bytes of one row handled by one comm unit
 constexpr int kPermUnitRows = 32;      // rows of one permute unit of MoE layer 0 (32 rows x 2 KB by the 128 comm threads)
 constexpr int kPermUnitsPerSlice = kBM / kPermUnitRows;
+constexpr int kPermBlockRows = 256;    // sorted rows per counter of the destination-order permute
 constexpr int kGrTokBlock = 32;        // tokens per combine / reduce work item of MoE layer 1
 constexpr int kAgMaxGroups = 64;       // arrival counters per (source rank, chunk): one per group of 2 KB slices
 
@@ -148,6 +149,10 @@ struct GemmParams {
   // an expert-sorted buffer (which tmap_a then describes) and count finished work items per source rank
   uint8_t* g_sorted;              // [rows, K] sorted activations, null = gather4 form
   int* g_perm_done;               // [world * g_nvr] finished permute units per source block (local, zeroed per call)
+  // destination order (one rank): row -> token of the sorted order. The comm warps then fill the sorted buffer row by
+  // row, g_perm_done counts the finished units of every block of kPermBlockRows sorted rows, and a tile waits for
+  // the blocks it overlaps only; null = source order
+  const int* g_perm_src;
   int g_vblk, g_nvr;              // tokens per source block (a multiple of 128) and blocks per rank (world * g_nvr <= 32)
   const int* g_scatter_index;     // [tokens, topk]
   const int* g_row_range;         // device [2]: rows [lo, hi) of the sorted order that this rank computes (expert
@@ -533,7 +538,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
   const int perm_units = perm_nvr * perm_slots;
   // step 0 (this rank's own tokens, nothing to wait for) gates the first tiles: the epilogue warps, idle until
   // the first accumulator is complete, permute every second unit of it
-  const bool perm_helped = p.g_sorted != nullptr && (p.ag_flags == nullptr || p.g_tokens_own != nullptr);
+  const bool perm_helped = p.g_sorted != nullptr && p.g_perm_src == nullptr && (p.ag_flags == nullptr || p.g_tokens_own != nullptr);
   auto permute_unit = [&](auto bar_tag, int u, int src_rank, int tid, bool may_wait) -> bool {
     constexpr int BAR = decltype(bar_tag)::value;
     const long long tok0 = static_cast<long long>(src_rank) * p.g_rows_per_rank;
@@ -609,6 +614,50 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     asm volatile("bar.sync %0, 128;" ::"n"(BAR) : "memory");
     if (tid == 0) red_add_release_gpu(p.g_perm_done + src_rank * perm_nvr + vb, 1);
     return true;
+  };
+
+  // Destination order (one rank, nothing to wait for): unit = 32 rows of the sorted buffer x one 2 KB slice, row groups
+  // first, so that the rows of the first tiles are in place after a few microseconds and the rest is copied while the
+  // GEMM runs. (In source order the first tile waited for all rows: 67 of the 371 us of 8192 tokens x 4096, top-2,
+  // ffn 3584.) The epilogue warps, idle until the first accumulators are complete, take every second unit of the
+  // rows that the first wave of tiles reads.
+  const int dst_groups = (p.M + kPermUnitRows - 1) / kPermUnitRows;
+  const int dst_units = dst_groups * ag_nslices;
+  int dst_shared = 0;  // units shared between the comm and the epilogue warps
+  if (p.g_perm_src != nullptr) {
+    const int wave_tiles = (tile_step + n_tiles - 1) / n_tiles;
+    const int bands = (wave_tiles + p.group_m - 1) / p.group_m;
+    const long long wave_units = static_cast<long long>(bands) * p.group_m * (TILE_M / kPermUnitRows) * ag_nslices;
+    dst_shared = wave_units < dst_units ? static_cast<int>(wave_units) : dst_units;
+  }
+  auto permute_dst_unit = [&](auto bar_tag, int u, int tid) {
+    constexpr int BAR = decltype(bar_tag)::value;
+    const int grp = u / ag_nslices;
+    const int ks = u - grp * ag_nslices;
+    const int r0 = grp * kPermUnitRows;
+    const int nrows = imin(kPermUnitRows, p.M - r0);
+    const long long b0 = static_cast<long long>(ks) * kCommSliceBytes + tid * 16;
+    const bool active = b0 < p.ag_row_bytes;
+    const int mine = lane < nrows ? p.g_perm_src[r0 + lane] : -1;
+    uint8_t* d0 = p.g_sorted + static_cast<long long>(r0) * p.ag_row_bytes + b0;
+#pragma unroll 1
+    for (int rr = 0; rr < nrows; rr += 16) {
+      uint4 val[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int tok = __shfl_sync(0xffffffffu, mine, rr + j);
+        // (a corrupt routing table must not become a wild load)
+        if (active && tok >= 0 && tok < p.g_ntokens)
+          val[j] = __ldg(reinterpret_cast<const uint4*>(p.g_tokens + static_cast<long long>(tok) * p.ag_row_bytes + b0));
+        else
+          val[j] = make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (active && rr + j < nrows) *reinterpret_cast<uint4*>(d0 + (rr + j) * p.ag_row_bytes) = val[j];
+    }
+    asm volatile("bar.sync %0, 128;" ::"n"(BAR) : "memory");
+    if (tid == 0) red_add_release_gpu(p.g_perm_done + r0 / kPermBlockRows, 1);
   };
 
   // Abort path of the producer: every stage it armed still has copies in flight or has been filled; wait
@@ -697,6 +746,12 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
           const int cpv = (p.g_vblk > 0 ? p.g_vblk : p.g_rows_per_rank + kBM - 1) / kBM;  // chunks per block
           const int all_chunks = (p.g_rows_per_rank + kBM - 1) / kBM;
           const uint64_t w0 = tr != nullptr ? globaltimer_ns() : 0;
+          if (p.g_perm_src != nullptr) {
+            for (int b = tc.row0 / kPermBlockRows; ok && tc.rows > 0 && b * kPermBlockRows < tc.row0 + tc.rows; ++b) {
+              const int groups = (imin(kPermBlockRows, p.M - b * kPermBlockRows) + kPermUnitRows - 1) / kPermUnitRows;
+              ok = flag_wait_eq(p.g_perm_done + b, groups * ag_nslices, ab, kStatusTimeoutFlag, budget);
+            }
+          } else
           for (int b = 0; ok && b < p.world * nvr; ++b)
             if ((tc.need_mask >> b) & 1) {
               const int j = b % nvr;
@@ -865,6 +920,9 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       for (int u = cta_id + num_ctas; u < perm_units; u += 2 * num_ctas)
         permute_unit(std::integral_constant<int, 2>{}, u, p.rank, static_cast<int>(threadIdx.x) - 2 * 32, false);
     }
+    if (p.g_perm_src != nullptr)
+      for (int u = cta_id + num_ctas; u < dst_shared; u += 2 * num_ctas)
+        permute_dst_unit(std::integral_constant<int, 2>{}, u, static_cast<int>(threadIdx.x) - 2 * 32);
     int it = 0;
     int t, kb0, kb1, part;
     for (; get_item(it, t, kb0, kb1, part); ++it) {
@@ -1405,7 +1463,14 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     // to the rank that needs it d-th soonest (rank-1, rank-2, ...; one destination at a time, so every link
     // carries one stream at full rate and shards land in the order they are consumed).
     // The push is skipped when the copy engines carry the all-gather (p.ag_src == nullptr).
-    if (p.ag_src != nullptr || p.g_sorted != nullptr) {
+    if (p.g_perm_src != nullptr) {
+      const int ctid = threadIdx.x - 6 * 32;  // 0..127
+      int u = cta_id;
+      for (; u < dst_shared; u += 2 * num_ctas) permute_dst_unit(std::integral_constant<int, 1>{}, u, ctid);
+      // the rest, units dst_shared and up, by the comm warps alone
+      for (u = dst_shared + (cta_id + num_ctas - dst_shared % num_ctas) % num_ctas; u < dst_units; u += num_ctas)
+        permute_dst_unit(std::integral_constant<int, 1>{}, u, ctid);
+    } else if (p.ag_src != nullptr || p.g_sorted != nullptr) {
       const int ctid = threadIdx.x - 6 * 32;  // 0..127
       // own rows are read from the caller's tensor (dense: by the own tiles; MoE: by the permute): no copy to itself
       const int d_first = (p.ag_src != nullptr && (p.a_own_valid || p.g_tokens_own != nullptr)) ? 1 : 0;

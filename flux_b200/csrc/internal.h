@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdarg.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <functional>
 #include <string>
@@ -35,6 +36,33 @@ void set_error(const char* fmt, ...);
       FLUXB_FAIL(FLUXB_ERR_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e_), \
                  __FILE__, __LINE__);                                                 \
   } while (0)
+
+// Launches with the programmatic-dependent-launch attribute: the kernel must call pdl_wait() before it touches global
+// memory, and pdl_trigger() for the next one to be let in early.
+template <class... P, class... A>
+inline int launch_pdl_cluster(void (*kern)(P...), int grid, int threads, size_t smem, int cluster, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+  return FLUXB_OK;
+}
+template <class... P, class... A>
+inline int launch_pdl(void (*kern)(P...), int grid, int threads, cudaStream_t stream, A... args) {
+  return launch_pdl_cluster(kern, grid, threads, 0, 0, stream, args...);
+}
 
 inline int dtype_bytes(int dt) {
   switch (dt) {

@@ -7,8 +7,6 @@
 // (src/cuda/moe_utils.cu:23-75) orders rows inside an expert with shared
 // memory atomics; this one does not.
 // gather index: inverse permutation (src/moe_ag_scatter/sort_util.cu:39-92).
-#include <string.h>
-
 #include "internal.h"
 
 namespace fluxb {
@@ -133,29 +131,6 @@ __global__ void gather_index_kernel(const int* __restrict__ scatter_index, int t
   if (topk_index != nullptr) topk_index[row] = i % topk;
 }
 
-// Launch with a cluster dimension and the programmatic-dependent-launch attribute (the kernels above wait for the
-// previous one before they touch global memory).
-template <class... P, class... A>
-static int launch_small(void (*kern)(P...), int grid, int threads, size_t smem, int cluster, cudaStream_t stream, A... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-  return FLUXB_OK;
-}
-
 }  // namespace fluxb
 
 using namespace fluxb;
@@ -181,8 +156,8 @@ int fluxb_moe_scatter_index(const int* chosen_experts, int ntokens, int topk, in
   }
   // one CTA while its warps have a round of 32 pairs or two each, else the whole cluster
   const int ctas = total <= 2 * kIdxThreads ? 1 : kIdxCluster;
-  return launch_small(scatter_index_kernel, ctas, kIdxThreads, idx_smem_bytes(nexperts), ctas, static_cast<cudaStream_t>(stream),
-                      chosen_experts, static_cast<int>(total), nexperts, splits_out, scatter_index_out);
+  return launch_pdl_cluster(scatter_index_kernel, ctas, kIdxThreads, idx_smem_bytes(nexperts), ctas,
+                            static_cast<cudaStream_t>(stream), chosen_experts, static_cast<int>(total), nexperts, splits_out, scatter_index_out);
 }
 
 int fluxb_moe_gather_index(const int* scatter_index, int ntokens, int topk, int* gather_index_out,
@@ -193,8 +168,8 @@ int fluxb_moe_gather_index(const int* scatter_index, int ntokens, int topk, int*
   FLUXB_REQUIRE(total < (1ll << 30), "moe_gather_index: too many routed rows");
   if (total == 0) return FLUXB_OK;
   const int blocks = static_cast<int>((total + 255) / 256);
-  return launch_small(gather_index_kernel, blocks, 256, 0, 1, static_cast<cudaStream_t>(stream), scatter_index,
-                      static_cast<int>(total), topk, gather_index_out, topk_index_out);
+  return launch_pdl(gather_index_kernel, blocks, 256, static_cast<cudaStream_t>(stream), scatter_index,
+                    static_cast<int>(total), topk, gather_index_out, topk_index_out);
 }
 
 }  // extern "C"

@@ -133,6 +133,145 @@ __global__ void moe_route_rows_kernel(const int* __restrict__ scatter_index, int
   atomicOr(&t.tiles[tile].need_mask, 1 << (src * nvr + (token - src * tokens_per_rank) / vblk));
 }
 
+// Tile list of up to 1024 experts by one block of 1024 threads, thread e with expert e's rows: prefixes by warp scans.
+__device__ __forceinline__ void write_tile_table(int split, int total_rows, int max_tiles, int tile_m, const MoeTables& t,
+                                                 int* status) {
+  __shared__ int2 warp_sum[32];
+  __shared__ int2 s_all;
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+  const int n = split < 0 ? 0 : split;
+  const int nt = (n + tile_m - 1) / tile_m;
+  int rows = n, tiles = nt;  // inclusive prefixes
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int r = __shfl_up_sync(0xffffffffu, rows, off), q = __shfl_up_sync(0xffffffffu, tiles, off);
+    if (lane >= off) {
+      rows += r;
+      tiles += q;
+    }
+  }
+  if (lane == 31) warp_sum[warp] = make_int2(rows, tiles);
+  __syncthreads();
+  int row0 = rows - n, tile0 = tiles - nt;
+  for (int w = 0; w < warp; ++w) {
+    row0 += warp_sum[w].x;
+    tile0 += warp_sum[w].y;
+  }
+  if (e == 1023) {
+    s_all = make_int2(row0 + n, tile0 + nt);
+    const bool ok = row0 + n == total_rows && tile0 + nt <= max_tiles;
+    t.num_tiles[0] = ok ? tile0 + nt : 0;
+    t.num_tiles[1] = 0;
+    t.num_tiles[2] = total_rows;
+    if (!ok) {
+      *reinterpret_cast<volatile int*>(status) = kStatusBadTable;
+      __threadfence_system();
+    }
+  }
+  __syncthreads();
+  if (s_all.x != total_rows || s_all.y > max_tiles) return;
+  for (int c = 0; c < nt; ++c) {
+    GroupTile g;
+    g.a_row0 = row0 + c * tile_m;
+    g.rows = imin(tile_m, n - c * tile_m);
+    g.expert = e;
+    g.need_mask = 0;
+    t.tiles[tile0 + c] = g;
+  }
+}
+
+// One rank: tile list (block 0), row -> token of the sorted order (the other blocks) and the permute counters in one
+// launch; nothing in it depends on where a token comes from, so there are no masks.
+__global__ void __launch_bounds__(1024)
+moe_local_tables_kernel(const int* __restrict__ splits, const int* __restrict__ scatter_index, int nexperts, int total_rows,
+                        int topk, int max_tiles, int tile_m, int* perm_done, int perm_blocks, MoeTables t, int* status) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_trigger();
+  if (blockIdx.x > 0) {
+    const int i = (static_cast<int>(blockIdx.x) - 1) * 1024 + static_cast<int>(threadIdx.x);
+    if (i < total_rows) {
+      const int row = scatter_index[i];
+      if (row >= 0 && row < total_rows) t.gather[row] = i / topk;
+    }
+    return;
+  }
+  for (int b = threadIdx.x; b < perm_blocks; b += 1024) perm_done[b] = 0;
+  const int e = threadIdx.x;
+  write_tile_table(e < nexperts ? splits[e] : 0, total_rows, max_tiles, tile_m, t, status);
+}
+
+// The same table from splits the host knows, passed by value.
+struct HostSplits {
+  int v[1024];
+};
+__global__ void __launch_bounds__(1024)
+moe_host_tables_kernel(const __grid_constant__ HostSplits splits, int nexperts, int total_rows, int max_tiles, int tile_m,
+                       MoeTables t, int* status) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_trigger();
+  const int e = threadIdx.x;
+  write_tile_table(e < nexperts ? splits.v[e] : 0, total_rows, max_tiles, tile_m, t, status);
+}
+
+// out[t] = sum over k of d[scatter_index[t, k]], in fp32 in the order of k, rounded once: the combine of MoE layer 1 on
+// one rank. One thread = 8 columns of 4 tokens, so that up to 8 16-byte loads are in flight in each of 2048 threads
+// per SM. (Inside the GEMM's launch, 128 threads per SM summed column group by column group: 86 of the 443 us of 16384
+// rows x 4096 were left to do when the GEMM had ended, 117 of 243 with 8000 rows x 8192.)
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(const uint16_t* __restrict__ d, const int* __restrict__ scatter_index, uint16_t* __restrict__ out,
+                   int ntokens, int topk, int n, int rows, int is_bf16) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_trigger();
+  const int col = (static_cast<int>(blockIdx.y) * 64 + (static_cast<int>(threadIdx.x) & 63)) * 8;
+  const int t0 = (static_cast<int>(blockIdx.x) * 4 + (static_cast<int>(threadIdx.x) >> 6)) * 4;
+  if (col >= n) return;
+  float acc[4][8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
+  for (int k0 = 0; k0 < topk; k0 += 2) {
+    uint4 v[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[u][j] = make_uint4(0u, 0u, 0u, 0u);
+        if (k0 + u < topk && t0 + j < ntokens) {
+          const int row = scatter_index[static_cast<long long>(t0 + j) * topk + k0 + u];
+          if (row >= 0 && row < rows)  // a corrupt entry must not become a wild load
+            v[u][j] = __ldg(reinterpret_cast<const uint4*>(d + static_cast<long long>(row) * n + col));
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t w[4] = {v[u][j].x, v[u][j].y, v[u][j].z, v[u][j].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (is_bf16) {
+            acc[j][2 * i] += __uint_as_float(w[i] << 16);
+            acc[j][2 * i + 1] += __uint_as_float(w[i] & 0xFFFF0000u);
+          } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+            acc[j][2 * i] += f.x;
+            acc[j][2 * i + 1] += f.y;
+          }
+        }
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (t0 + j < ntokens) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        w[i] = is_bf16 ? pack_bf16(acc[j][2 * i], acc[j][2 * i + 1]) : pack_f16(acc[j][2 * i], acc[j][2 * i + 1]);
+      *reinterpret_cast<uint4*>(out + static_cast<long long>(t0 + j) * n + col) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 // Visiting order of the tiles: stable counting sort by how late the tile's last source block is permuted
 // (this rank's own blocks first, then rank+1's, ...), so that early tiles need early data.
 __global__ void moe_order_tiles_kernel(MoeTables t, int rank, int world, int nvr) {
@@ -177,6 +316,7 @@ struct fluxb_moe_ag_scatter {
   unsigned long long calls;
   int last_parity;      // parity of the buffers the last push filled
   int last_ntokens;     // tokens gathered by the last push
+  bool keep_tokens = true;  // one rank: calls with tokens leave a copy for calls without (tokens_shard == NULL)
   int ep_rank = 0, ep_size = 1;  // expert parallelism: this rank holds experts [ep_rank, ep_rank + 1) * nexperts / ep_size
   AgDma dma;
 };
@@ -200,10 +340,13 @@ static int flag_stride_of(int full_m, int world) {
 extern "C" {
 
 // ------------------------------------------------------------------ layer 0
+// permute counters: one per source block (at most 32), or one per kPermBlockRows sorted rows
+static size_t perm_counter_bytes(long long max_rows) { return align_up(static_cast<size_t>(max_rows / kPermBlockRows + 32) * sizeof(int), 256); }
+
 // [routing tables][permute counters][expert-sorted activations: max_ntokens*topk rows of `hidden` elements]
 size_t fluxb_moe_ag_scatter_workspace_bytes(int max_ntokens, int topk, int nexperts, int hidden, int in_dtype) {
   const long long rows = static_cast<long long>(max_ntokens) * topk;
-  return tables_bytes(rows, nexperts) + 256 +
+  return tables_bytes(rows, nexperts) + perm_counter_bytes(rows) +
          align_up(static_cast<size_t>(rows + kBM) * hidden * dtype_bytes(in_dtype), 256);
 }
 
@@ -271,6 +414,14 @@ int fluxb_moe_ag_scatter_set_ep(fluxb_moe_ag_scatter_t op, int ep_rank, int ep_s
   return FLUXB_OK;
 }
 
+int fluxb_moe_ag_scatter_keep_tokens(fluxb_moe_ag_scatter_t op, int keep) {
+  FLUXB_REQUIRE(op != nullptr, "moe_ag_scatter_keep_tokens: op is NULL");
+  FLUXB_REQUIRE(keep != 0 || op->comm->world == 1, "moe_ag_scatter_keep_tokens: with several ranks the gathered tokens are always kept");
+  op->keep_tokens = keep != 0;
+  op->last_parity = -1;
+  return FLUXB_OK;
+}
+
 int fluxb_moe_ag_scatter_reset(fluxb_moe_ag_scatter_t op, fluxb_stream_t stream) {
   FLUXB_REQUIRE(op != nullptr, "moe_ag_scatter_reset: op is NULL");
   FLUXB_CUDA(cudaMemsetAsync(op->flags[op->comm->rank], 0, fluxb_ag_gemm_flag_bytes(op->max_ntokens, op->comm->world),
@@ -311,26 +462,41 @@ int fluxb_moe_ag_scatter_forward(fluxb_moe_ag_scatter_t op, const void* tokens_s
   const int cg = grouped_cta_group(tuning, rows, op->nexperts);
   const int tile_m = cg == 2 ? 2 * kBM : kBM;
   const int e_count = op->nexperts / op->ep_size, e_first = op->ep_rank * e_count;
-  moe_build_tiles_kernel<<<1, 1024, 0, stream>>>(splits_dev, op->nexperts, e_first, e_count, static_cast<int>(rows),
-                                                max_tiles, tile_m, tb, comm->status_dev);
-  FLUXB_CUDA(cudaGetLastError());
-  // source blocks of about 1024 tokens (whole 128-token chunks), at most 32 over all ranks: a 256-row tile of an
-  // expert spans about that many tokens, so it can start when a fraction of a rank's tokens is in place
-  // (only while all experts' weights fit in L2: visiting tiles block by block instead of expert by expert
-  // re-streams every expert's weights once per block - measured at TP=1, 940 MB of weights: 1.85 ms against 1.58)
-  int nvr = ntokens_local / 1024;
-  if (nvr > 32 / world) nvr = 32 / world;
-  if (static_cast<double>(e_count) * op->ffn_local * row_bytes > 64.0 * 1024 * 1024) nvr = 1;
-  if (nvr < 1) nvr = 1;
-  const int vblk = ((ntokens_local + nvr - 1) / nvr + kBM - 1) / kBM * kBM;
-  nvr = (ntokens_local + vblk - 1) / vblk;
-  moe_route_rows_kernel<<<static_cast<int>((rows + 255) / 256), 256, 0, stream>>>(
-      scatter_index_dev, static_cast<int>(rows), op->topk, ntokens_local, vblk, nvr, op->nexperts, tile_m, tb);
-  FLUXB_CUDA(cudaGetLastError());
-  if (world * nvr > 1) {
-    moe_order_tiles_kernel<<<1, 32, 0, stream>>>(tb, comm->rank, world, nvr);
+  uint8_t* ws = static_cast<uint8_t*>(op->workspace);
+  int* perm_done = reinterpret_cast<int*>(ws + tables_bytes(max_rows, op->nexperts));
+  int vblk = ntokens_local, nvr = 1;
+  // one rank, nothing arrives: the sorted buffer is filled in destination order (see GemmParams::g_perm_src)
+  const bool local = world == 1 && comm->ranks_on_gpu <= 1;
+  if (local) {
+    const int perm_blocks = static_cast<int>((rows + kPermBlockRows - 1) / kPermBlockRows);
+    int rc0 = launch_pdl(moe_local_tables_kernel, 1 + static_cast<int>((rows + 1023) / 1024), 1024, stream, splits_dev,
+                         scatter_index_dev, op->nexperts, static_cast<int>(rows), op->topk, max_tiles, tile_m, perm_done,
+                         perm_blocks, tb, comm->status_dev);
+    if (rc0 != FLUXB_OK) return rc0;
+    p.g_perm_src = tb.gather;
+  } else {
+    moe_build_tiles_kernel<<<1, 1024, 0, stream>>>(splits_dev, op->nexperts, e_first, e_count, static_cast<int>(rows),
+                                                  max_tiles, tile_m, tb, comm->status_dev);
     FLUXB_CUDA(cudaGetLastError());
-    p.g_order = tb.order;
+    // source blocks of about 1024 tokens (whole 128-token chunks), at most 32 over all ranks: a 256-row tile of an
+    // expert spans about that many tokens, so it can start when a fraction of a rank's tokens is in place
+    // (only while all experts' weights fit in L2: visiting tiles block by block instead of expert by expert
+    // re-streams every expert's weights once per block - measured at TP=1, 940 MB of weights: 1.85 ms against 1.58)
+    nvr = ntokens_local / 1024;
+    if (nvr > 32 / world) nvr = 32 / world;
+    if (static_cast<double>(e_count) * op->ffn_local * row_bytes > 64.0 * 1024 * 1024) nvr = 1;
+    if (nvr < 1) nvr = 1;
+    vblk = ((ntokens_local + nvr - 1) / nvr + kBM - 1) / kBM * kBM;
+    nvr = (ntokens_local + vblk - 1) / vblk;
+    moe_route_rows_kernel<<<static_cast<int>((rows + 255) / 256), 256, 0, stream>>>(
+        scatter_index_dev, static_cast<int>(rows), op->topk, ntokens_local, vblk, nvr, op->nexperts, tile_m, tb);
+    FLUXB_CUDA(cudaGetLastError());
+    if (world * nvr > 1) {
+      moe_order_tiles_kernel<<<1, 32, 0, stream>>>(tb, comm->rank, world, nvr);
+      FLUXB_CUDA(cudaGetLastError());
+      p.g_order = tb.order;
+    }
+    FLUXB_CUDA(cudaMemsetAsync(perm_done, 0, 256, stream));
   }
   p.g_vblk = vblk;
   p.g_nvr = nvr;
@@ -369,11 +535,8 @@ int fluxb_moe_ag_scatter_forward(fluxb_moe_ag_scatter_t op, const void* tokens_s
   p.g_scatter_index = scatter_index_dev;
   p.g_row_range = tb.num_tiles + 1;  // rows of this rank's experts (all rows without expert parallelism)
   p.ag_row_bytes = row_bytes;
-  uint8_t* ws = static_cast<uint8_t*>(op->workspace);
-  int* perm_done = reinterpret_cast<int*>(ws + tables_bytes(max_rows, op->nexperts));
   p.g_perm_done = perm_done;
-  p.g_sorted = ws + tables_bytes(max_rows, op->nexperts) + 256;
-  FLUXB_CUDA(cudaMemsetAsync(perm_done, 0, 256, stream));
+  p.g_sorted = ws + tables_bytes(max_rows, op->nexperts) + perm_counter_bytes(max_rows);
   uint8_t* local_gather = op->gather[comm->rank] + parity * half_gather;
   if (world == 1 && !reuse) {
     p.g_tokens = static_cast<const uint8_t*>(tokens_shard);  // nothing to gather: permute straight from the caller's tokens
@@ -417,6 +580,12 @@ int fluxb_moe_ag_scatter_forward(fluxb_moe_ag_scatter_t op, const void* tokens_s
   rc = launch_fused_gemm(comm, p, op->in_dtype, &t, stream);
   if (rc != FLUXB_OK) return rc;
   if (dma) FLUXB_CUDA(cudaStreamWaitEvent(stream, op->dma.ev_done, 0));
+  if (!reuse && !op->keep_tokens) {
+    op->calls += 1;
+    if (gathered_out != nullptr)  // one rank: its tokens are all tokens
+      FLUXB_CUDA(cudaMemcpyAsync(gathered_out, tokens_shard, static_cast<size_t>(ntokens) * row_bytes, cudaMemcpyDeviceToDevice, stream));
+    return FLUXB_OK;
+  }
   if (!reuse) {
     // keep a copy of the own tokens in the gather buffer (after the launch, off its critical path) so that
     // further weight groups and `gathered_out` find every rank's tokens there
@@ -586,8 +755,20 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
   void* inter = ws;
   MoeTables tb = carve_tables(ws + align_up(static_cast<size_t>(op->max_m) * n * 2, 256), op->max_m, op->nexperts);
   const int num_tiles = static_cast<int>(tiles.size());
-  FLUXB_CUDA(cudaMemcpyAsync(tb.tiles, tiles.data(), tiles.size() * sizeof(GroupTile), cudaMemcpyHostToDevice, stream));
-  FLUXB_CUDA(cudaMemcpyAsync(tb.num_tiles, &num_tiles, sizeof(int), cudaMemcpyHostToDevice, stream));
+  // one rank: the table comes from a kernel that gets the splits by value, the GEMM only stores its rows, and the combine
+  // is a launch of its own
+  const bool local = world == 1 && comm->ranks_on_gpu <= 1;
+  if (local) {
+    HostSplits hs;
+    memcpy(hs.v, splits_host, static_cast<size_t>(op->nexperts) * sizeof(int));
+    memset(hs.v + op->nexperts, 0, (1024 - static_cast<size_t>(op->nexperts)) * sizeof(int));
+    const int rc0 = launch_pdl(moe_host_tables_kernel, 1, 1024, stream, hs, op->nexperts, static_cast<int>(rows_all),
+                               num_tiles, tile_m, tb, comm->status_dev);
+    if (rc0 != FLUXB_OK) return rc0;
+  } else {
+    FLUXB_CUDA(cudaMemcpyAsync(tb.tiles, tiles.data(), tiles.size() * sizeof(GroupTile), cudaMemcpyHostToDevice, stream));
+    FLUXB_CUDA(cudaMemcpyAsync(tb.num_tiles, &num_tiles, sizeof(int), cudaMemcpyHostToDevice, stream));
+  }
 
   p.out_type = op->out_dtype == FLUXB_BF16 ? kOutBf16 : kOutF16;
   p.M = m > 0 ? m : 1;
@@ -616,6 +797,27 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
                       cg == 2 ? bn / 2 : bn);
   if (rc != FLUXB_OK) return rc;
   encode_out_map(p, inter, p.M, n, p.out_type);
+  if (local) {
+    fluxb_tuning tl = tuning != nullptr ? *tuning : fluxb_tuning{0, 0, 0, 0, 0};
+    tl.block_n = bn;
+    tl.cta_group = cg;
+    rc = launch_fused_gemm(comm, p, op->in_dtype, &tl, stream);
+    if (rc != FLUXB_OK) return rc;
+    op->calls += 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(static_cast<unsigned>((ntokens + 15) / 16), static_cast<unsigned>((n / 8 + 63) / 64), 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FLUXB_CUDA(cudaLaunchKernelEx(&cfg, moe_combine_kernel, static_cast<const uint16_t*>(inter), routing_idx_dev,
+                                  static_cast<uint16_t*>(out), ntokens, topk, n, m, op->out_dtype == FLUXB_BF16 ? 1 : 0));
+    return FLUXB_OK;
+  }
   // combine + reduce-scatter run inside the same launch (comm warps), column slab by column slab
   const int parity = static_cast<int>(op->calls & 1ull);
   const size_t half_stage_elems = (static_cast<size_t>(op->max_m) / topk) * n;

@@ -90,6 +90,8 @@ class GemmGroupedV3AGScatter:
         self._h = h
         if self.ep_size > 1:
             _lib.check(lib.fluxb_moe_ag_scatter_set_ep(h, self.ep_rank, self.ep_size))
+        if w == 1:  # every call below brings its tokens along
+            _lib.check(lib.fluxb_moe_ag_scatter_keep_tokens(h, 0))
         self.comm.host_barrier()
 
     def __del__(self):
@@ -166,7 +168,7 @@ class GemmGroupedV3AGScatter:
                 inputs_shard, wt, splits_gpu, scatter_index,
                 None if output_scale is None else output_scale[i],
                 None if outputs_buf is None else outputs_buf[i],
-                allgather_output if i == 0 else None, tuning, reuse=(i > 0)))
+                allgather_output if i == 0 else None, tuning, reuse=(i > 0 and self.comm.world > 1)))
         return outs
 
     def clear_buffers(self):

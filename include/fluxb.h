@@ -225,6 +225,9 @@ int fluxb_moe_ag_scatter_reset(fluxb_moe_ag_scatter_t op, fluxb_stream_t stream)
  * `out` receives only the rows of this rank's experts, numbered from the first of them
  * (python/flux/testing/moe_ag_scatter_utils.py:228-262). */
 int fluxb_moe_ag_scatter_set_ep(fluxb_moe_ag_scatter_t op, int ep_rank, int ep_size);
+/* One rank only: `keep` = 0 promises that every forward call brings its tokens (tokens_shard != NULL), which saves the
+ * copy of them that a later call without tokens would read; such a call is then refused. Default 1. */
+int fluxb_moe_ag_scatter_keep_tokens(fluxb_moe_ag_scatter_t op, int keep);
 int fluxb_moe_ag_scatter_forward(fluxb_moe_ag_scatter_t op, const void* tokens_shard,
                                  int ntokens_local, const void* weights, const int* splits_dev,
                                  const int* scatter_index_dev, const float* out_scale, void* out,
