@@ -78,7 +78,6 @@ struct GemmParams {
   int tmap_out_valid;
   int a_own_valid;
   int b_mn_major;  // 1: B is stored [K, N] (N contiguous), loaded as 64-column boxes (16-bit inputs only)
-  int acc_int;     // 1: 8-bit operands are signed integers and the accumulator is int32 (w8a8 with dequantisation)
   int M, N, K;
   // M segmentation: nseg segments of seg_rows rows; tiles never straddle a
   // segment; segments are visited (seg_first + i) % nseg.
@@ -400,7 +399,9 @@ __device__ __forceinline__ void add_parked(uint32_t (&r)[32], const float* src, 
   }
 }
 
-// KIND: 0 = 16-bit inputs (bf16/f16 chosen by the instruction descriptor), 1 = fp8
+// KIND: 0 = 16-bit inputs (bf16/f16 chosen by the instruction descriptor), 1 = fp8, 2 = int8 with int32 accumulators (w8a8
+// with dequantisation). A choice between the last two at run time put a branch around every UMMA: 375 ns per K block
+// instead of the 276 that a 256 x 256 tile's UMMAs take.
 // CTA2: false = one CTA per 128-row tile, true = CTA pair per 256-row tile (launch with cluster 2x1x1)
 // `cta_id` / `num_ctas`: this CTA's index and the number of CTAs that work on problem `p` (the whole grid for
 // an ordinary launch; a slice of it when one launch runs several ranks' problems side by side).
@@ -846,7 +847,6 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     // ----------------------------------------------------------------- UMMA
     if (leader && elect_one()) {  // see the note on elect.sync above
       const bool b_kn = p.b_mn_major != 0;
-      const bool acc_int = KIND == 1 && p.acc_int;
       // Operand descriptors of stage 0; a later stage only moves the start address (bits [0,14), in units of 16 B).
       // Each UMMA consumes 32 bytes of K of a K-major operand: advance the start address by 32 B
       // (>>4 = 2); of an MN-major operand it consumes 16 K rows of 128 B: 2048 B (>>4 = 128)
@@ -880,11 +880,11 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
             const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
             if (CTA2) {
               if (KIND == 0) umma_f16_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
-              else if (acc_int) umma_i8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
+              else if (KIND == 2) umma_i8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
               else umma_f8_2cta(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
             } else {
               if (KIND == 0) umma_f16(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
-              else if (acc_int) umma_i8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
+              else if (KIND == 2) umma_i8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
               else umma_f8(d_tmem, a_desc + 2u * k, b_desc + b_step * k, idesc, accum);
             }
           }
@@ -1075,7 +1075,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
                         (p.bias_mode == kBiasNone || ((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0 && (p.ldbias & 7) == 0)) &&
                         (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
       if (lean) {
-        const bool acc_int = KIND == 1 && p.acc_int;
+        constexpr bool acc_int = KIND == 2;
         const bool to_bf16 = otype == kOutBf16;
         const float* sb_ptr = p.scale_b;
         const bool has_bias = p.bias_mode != kBiasNone;
@@ -1198,9 +1198,9 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         tmem_ld_wait();
         const int col0 = tc.n0 + c * 32;
         const bool active = row_ok && col0 < p.N;
-        if (is_tail) add_parked(r, sk_warp + c * (8 * 32 * 4), TILE_M * BN, split - 1, KIND == 1 && p.acc_int);
+        if (is_tail) add_parked(r, sk_warp + c * (8 * 32 * 4), TILE_M * BN, split - 1, KIND == 2);
         float v[32];
-        if (KIND == 1 && p.acc_int) {
+        if (KIND == 2) {
           // int8 operands, int32 accumulator. Dequantisation in the reference's order, so that the result is
           // bit-identical to its golden path (test/python/ag_gemm/test_ag_kernel.py:143-150, threshold 0):
           // (input_scale[row] * weight_scale[col]) * float(acc), rounded to the 16-bit output; a bias is then
@@ -1250,7 +1250,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
             }
           }
         }
-        if (own && active && (p.rs_ring || (KIND == 1 && p.acc_int))) {
+        if (own && active && (p.rs_ring || KIND == 2)) {
           // ring order: the own partial joins last, as a 16-bit value like the peers'; w8a8: every rank's
           // dequantised partial is a 16-bit tensor in the reference (test/python/gemm_rs/test_gemm_rs.py:127-135)
 #pragma unroll

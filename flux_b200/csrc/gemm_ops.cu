@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "plain_gemm.cuh"
 #include "skinny_gemm.cuh"
 
 namespace fluxb {
@@ -246,16 +247,14 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
   p.splitk_done = comm->splitk_cnt + comm->sm_count * 8;
   p.rank = comm->rank;
   p.world = comm->world;
-  const int kind = is_8bit(in_dtype) ? 1 : 0;
+  const int kind = kind_of(in_dtype);
   uint32_t fmt;
   const int rc_fmt = input_format(in_dtype, &fmt);
   if (rc_fmt != FLUXB_OK) return rc_fmt;
-  p.acc_int = is_int8(in_dtype) ? 1 : 0;
-  if (p.acc_int) {
+  if (is_int8(in_dtype))
     FLUXB_REQUIRE(p.out_type != kOutF32 || p.epi_mode == kEpiRsPush, "int8 inputs produce a 16-bit output");
-  }
   const uint32_t idesc = make_idesc(fmt, cg == 2 ? 2 * kBM : kBM, static_cast<uint32_t>(bn), p.b_mn_major ? 1u : 0u,
-                                    p.acc_int ? 2u : 1u);
+                                    is_int8(in_dtype) ? 2u : 1u);
   if (comm->ranks_on_gpu > 1) {
     DeferredItem it;
     it.fused = true;
@@ -268,11 +267,11 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
     comm->deferred.push_back(std::move(it));
     return FLUXB_OK;
   }
-#define FLUXB_LAUNCH(BN_, ST1_, ST2_)                                                              \
-  (cg == 2 ? (kind == 0 ? launch_inst<BN_, ST2_, 0, true>(comm, p, idesc, grid, stream)            \
-                        : launch_inst<BN_, ST2_, 1, true>(comm, p, idesc, grid, stream))           \
-           : (kind == 0 ? launch_inst<BN_, ST1_, 0, false>(comm, p, idesc, grid, stream)           \
-                        : launch_inst<BN_, ST1_, 1, false>(comm, p, idesc, grid, stream)))
+#define FLUXB_LAUNCH_KIND(BN_, ST_, CTA2_)                                             \
+  (kind == 0 ? launch_inst<BN_, ST_, 0, CTA2_>(comm, p, idesc, grid, stream)           \
+   : kind == 1 ? launch_inst<BN_, ST_, 1, CTA2_>(comm, p, idesc, grid, stream)         \
+               : launch_inst<BN_, ST_, 2, CTA2_>(comm, p, idesc, grid, stream))
+#define FLUXB_LAUNCH(BN_, ST1_, ST2_) (cg == 2 ? FLUXB_LAUNCH_KIND(BN_, ST2_, true) : FLUXB_LAUNCH_KIND(BN_, ST1_, false))
   switch (bn) {
     case 256: return FLUXB_LAUNCH(256, stages_for(256, false), stages_for(256, true));
     case 192: return FLUXB_LAUNCH(192, stages_for(192, false), stages_for(192, true));
@@ -280,6 +279,7 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
     default: return FLUXB_LAUNCH(64, stages_for(64, false), stages_for(64, true));
   }
 #undef FLUXB_LAUNCH
+#undef FLUXB_LAUNCH_KIND
 }
 
 // ---------------------------------------------------------------------------
@@ -355,7 +355,6 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
   p.N = n;
   p.num_kb = static_cast<int>((row_bytes + kRowBytes - 1) / kRowBytes);
   p.w_kn = (flags & FLUXB_WEIGHT_KN) ? 1 : 0;
-  p.acc_int = is_int8(in_dtype) ? 1 : 0;
   p.out_bf16 = out_type == kOutBf16 ? 1 : 0;
   p.bias_mode = bias_mode;
   p.out = static_cast<uint16_t*>(c);
@@ -380,12 +379,15 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
   uint32_t fmt;
   rc = input_format(in_dtype, &fmt);
   if (rc != FLUXB_OK) return rc;
-  const uint32_t idesc = make_idesc(fmt, kBM, static_cast<uint32_t>(bn), 0u, p.acc_int ? 2u : 1u, p.w_kn ? 1u : 0u);
+  const uint32_t idesc = make_idesc(fmt, kBM, static_cast<uint32_t>(bn), 0u, is_int8(in_dtype) ? 2u : 1u, p.w_kn ? 1u : 0u);
   const int n_tiles = (n + kBM - 1) / kBM;
   p.split = skinny_split(comm->sm_count, n_tiles, p.num_kb, bn);
   const int grid = n_tiles * p.split;
-#define FLUXB_SKINNY(BN_) \
-  (is_8bit(in_dtype) ? launch_skinny_inst<BN_, 1>(p, idesc, grid, stream) : launch_skinny_inst<BN_, 0>(p, idesc, grid, stream))
+  const int kind = kind_of(in_dtype);
+#define FLUXB_SKINNY(BN_)                                                    \
+  (kind == 0 ? launch_skinny_inst<BN_, 0>(p, idesc, grid, stream)            \
+   : kind == 1 ? launch_skinny_inst<BN_, 1>(p, idesc, grid, stream)          \
+               : launch_skinny_inst<BN_, 2>(p, idesc, grid, stream))
   switch (bn) {
     case 16: return FLUXB_SKINNY(16);
     case 32: return FLUXB_SKINNY(32);
@@ -394,6 +396,141 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
     default: return FLUXB_SKINNY(256);
   }
 #undef FLUXB_SKINNY
+}
+
+// ---------------------------------------------------------------------------
+// plain GEMM (plain_gemm.cuh)
+// ---------------------------------------------------------------------------
+template <int BN, int KIND, bool CTA2>
+static int launch_plain_inst(const fluxb_comm* comm, PlainParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+  using L = PlainLayout<BN, CTA2>;
+  auto kern = plain_gemm_kernel<BN, KIND, CTA2>;
+  static bool configured[64] = {};
+  static int max_clusters[64] = {};
+  int dev = 0;
+  FLUXB_CUDA(cudaGetDevice(&dev));
+  FLUXB_REQUIRE(dev < 64, "device index %d not supported", dev);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.blockDim = dim3(kPlainThreads, 1, 1);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CTA2 ? 2 : 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (!configured[dev]) {
+    FLUXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
+    if (CTA2) {
+      // how many CTA pairs can be resident at once: the persistent grid must not exceed it
+      cfg.gridDim = dim3(comm->sm_count & ~1, 1, 1);
+      int n = 0;
+      FLUXB_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+      FLUXB_REQUIRE(n >= 1, "no CTA pair of the plain kernel fits on this device");
+      max_clusters[dev] = n;
+    }
+    configured[dev] = true;
+  }
+  const int per = CTA2 ? 2 : 1;
+  int workers = grid / per;
+  if (CTA2 && workers > max_clusters[dev]) workers = max_clusters[dev];
+  if (workers < 1) workers = 1;
+  const int tiles = p.m_tiles * p.n_tiles;
+  if (workers > tiles) workers = tiles;
+  p.full_waves = tiles / workers;
+  p.tail_tiles = tiles - p.full_waves * workers;
+  p.split = splitk_parts(p.tail_tiles, workers, p.num_kb, false);
+  // the scratch holds 128 x 256 accumulators per SM: enough for any cut of tiles up to 256 columns, not of 512
+  while (p.split > 1 && static_cast<long long>(p.split - 1) * p.tail_tiles * per * BN > static_cast<long long>(comm->sm_count) * 256) --p.split;
+  p.split_div.set(static_cast<uint32_t>(p.split));
+  cfg.gridDim = dim3(workers * per, 1, 1);
+  cfg.numAttrs = 2;
+  FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, idesc));
+  return FLUXB_OK;
+}
+
+// 256 x 512 pair tiles instead of 256 x 256. They take a quarter less operand traffic per flop, which under the power cap
+// buys clock, but their epilogue (about 4 us) is not hidden: worth it from 128 K blocks on, with three waves or
+// more (the partial last wave is cut along K) and no column padding to speak of. Measured back to back for 0.4 s
+// (us, 256 / 512 columns): 4096 x 49152 x 12288 3640 / 3490, 4096 x 12288 x 49152 3700 / 3540, 8192 x 8192 x 8192 811 / 785, fp8
+// 8192 x 8192 x 16384 812 / 791; with 64 K blocks fp8 8192 x 28672 x 8192 1408 / 1425, 2048 x 14336 x 4096 180 / 183.
+static bool wide_tile_wins(int sm_count, int m, int n, long long row_bytes) {
+  const long long m_tiles = (m + 255) / 256, n_tiles = (n + 511) / 512;
+  return (row_bytes + kRowBytes - 1) / kRowBytes >= 128 && m_tiles * n_tiles >= 3ll * (sm_count / 2) && n_tiles * 512ll * 64 <= n * 65ll;
+}
+
+// 16-bit output; output, bias and column scales 16-byte aligned.
+static int launch_plain(const fluxb_comm* comm, const GemmParams& g, const void* a, const void* b, int in_dtype, int bn, int cg,
+                        const fluxb_tuning* tuning, cudaStream_t stream) {
+  FLUXB_REQUIRE(!g.b_mn_major || (bn / cg) % 64 == 0,
+                "a [K,N] weight needs a tile width whose per-CTA share is a multiple of 64 (block_n=%d, cta_group=%d)", bn, cg);
+  PlainParams p;
+  memset(&p, 0, sizeof(p));
+  const int eb = dtype_bytes(in_dtype);
+  const long long row_bytes = static_cast<long long>(g.K) * eb;
+  const int tile_m = cg * kBM;
+  p.M = g.M;
+  p.N = g.N;
+  p.num_kb = static_cast<int>((row_bytes + kRowBytes - 1) / kRowBytes);
+  p.n_tiles = (g.N + bn - 1) / bn;
+  p.m_tiles = (g.M + tile_m - 1) / tile_m;
+  FLUXB_REQUIRE(static_cast<long long>(p.n_tiles) * p.m_tiles < (1ll << 30), "gemm: %d x %d has too many tiles", g.M, g.N);
+  p.group_m = tuning != nullptr && tuning->group_m > 0 ? tuning->group_m : 8;
+  if (p.group_m > p.m_tiles) p.group_m = p.m_tiles;
+  p.band_div.set(static_cast<uint32_t>(p.group_m) * static_cast<uint32_t>(p.n_tiles));
+  p.gm_div.set(static_cast<uint32_t>(p.group_m));
+  p.last_div.set(static_cast<uint32_t>(p.m_tiles - (p.m_tiles - 1) / p.group_m * p.group_m));
+  p.b_kn = g.b_mn_major;
+  p.out_bf16 = g.out_type == kOutBf16 ? 1 : 0;
+  p.bias_mode = g.bias_mode;
+  p.alpha = g.alpha;
+  p.scale_a = g.scale_a;
+  p.scale_b = g.scale_b;
+  p.out = static_cast<uint16_t*>(g.out);
+  p.bias = static_cast<const uint16_t*>(g.bias);
+  p.splitk_scratch = comm->splitk_scratch;
+  p.splitk_cnt = comm->splitk_cnt;
+  p.splitk_done = comm->splitk_cnt + comm->sm_count * 8;
+  p.trace = comm->trace;
+  p.status = comm->status_dev;
+  p.timeout_ns = comm->timeout_ns;
+  int rc = encode_tmap_2d(&p.tmap_a, a, in_dtype, g.M, g.K, row_bytes, kBM);
+  if (rc != FLUXB_OK) return rc;
+  if (p.b_kn) {
+    FLUXB_REQUIRE(is_16bit(in_dtype), "a [K,N] weight needs 16-bit inputs (fp8 forbids transpose_weight)");
+    rc = encode_tmap_kn(&p.tmap_b, b, in_dtype, g.K, g.N, static_cast<long long>(g.N) * eb, kRowBytes / eb);
+  } else {
+    rc = encode_tmap_2d(&p.tmap_b, b, in_dtype, g.N, g.K, row_bytes, bn == 512 ? 128 : bn / cg);
+  }
+  if (rc != FLUXB_OK) return rc;
+  rc = encode_tmap_b16_store(&p.tmap_out, g.out, g.M, g.N);
+  if (rc != FLUXB_OK) return rc;
+  uint32_t fmt;
+  rc = input_format(in_dtype, &fmt);
+  if (rc != FLUXB_OK) return rc;
+  const uint32_t idesc = make_idesc(fmt, tile_m, static_cast<uint32_t>(bn == 512 ? 256 : bn), p.b_kn ? 1u : 0u, is_int8(in_dtype) ? 2u : 1u);
+  int grid = comm->sm_count;
+  if (tuning != nullptr && tuning->num_ctas > 0 && tuning->num_ctas < grid) grid = tuning->num_ctas;
+  const int kind = kind_of(in_dtype);
+#define FLUXB_PLAIN_KIND(BN_, CTA2_)                                                 \
+  (kind == 0 ? launch_plain_inst<BN_, 0, CTA2_>(comm, p, idesc, grid, stream)        \
+   : kind == 1 ? launch_plain_inst<BN_, 1, CTA2_>(comm, p, idesc, grid, stream)      \
+               : launch_plain_inst<BN_, 2, CTA2_>(comm, p, idesc, grid, stream))
+#define FLUXB_PLAIN(BN_) (cg == 2 ? FLUXB_PLAIN_KIND(BN_, true) : FLUXB_PLAIN_KIND(BN_, false))
+  switch (bn) {
+    case 512: return FLUXB_PLAIN_KIND(512, true);
+    case 256: return FLUXB_PLAIN(256);
+    case 192: return FLUXB_PLAIN(192);
+    case 128: return FLUXB_PLAIN(128);
+    default: return FLUXB_PLAIN(64);
+  }
+#undef FLUXB_PLAIN
+#undef FLUXB_PLAIN_KIND
 }
 
 static int out_type_of(int out_dtype, int* ot) {
@@ -509,7 +646,16 @@ int fluxb_gemm(fluxb_comm_t comm, const void* a, const void* b, void* c, int m, 
   p.scale_b = scale_b;
   p.alpha = alpha;
   p.b_mn_major = (flags & FLUXB_WEIGHT_KN) ? 1 : 0;
-  const int bn = resolve_block_n(comm, p, tuning, 0);
+  int bn = resolve_block_n(comm, p, tuning, 0);  // (the wide tile is not a caller's choice: it never was one)
+  if (comm->ranks_on_gpu <= 1 && p.out_type != kOutF32 &&
+      ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(bias_mode != FLUXB_BIAS_NONE ? bias : nullptr) |
+        reinterpret_cast<uintptr_t>(scale_b)) & 15) == 0) {
+    const int cg = resolve_cta_group(p, tuning);
+    FLUXB_REQUIRE(bn == 64 || bn == 128 || bn == 192 || bn == 256, "block_n=%d not in {64,128,192,256}", bn);
+    if (bn == 256 && cg == 2 && (tuning == nullptr || tuning->block_n == 0) && wide_tile_wins(comm->sm_count, m, n, static_cast<long long>(k) * eb))
+      bn = 512;
+    return launch_plain(comm, p, a, b, in_dtype, bn, cg, tuning, static_cast<cudaStream_t>(stream));
+  }
   rc = encode_tmap_2d(&p.tmap_a, a, in_dtype, m, k, static_cast<long long>(k) * eb, kBM);
   if (rc != FLUXB_OK) return rc;
   encode_out_map(p, c, m, n, p.out_type);

@@ -83,6 +83,7 @@ inline bool is_fp8(int dt) { return dt == FLUXB_E4M3 || dt == FLUXB_E5M2; }
 inline bool is_int8(int dt) { return dt == FLUXB_S8; }
 inline bool is_8bit(int dt) { return is_fp8(dt) || is_int8(dt); }
 inline bool is_16bit(int dt) { return dt == FLUXB_BF16 || dt == FLUXB_F16; }
+inline int kind_of(int dt) { return is_int8(dt) ? 2 : is_fp8(dt) ? 1 : 0; }  // KIND of the GEMM kernels
 
 }  // namespace fluxb
 

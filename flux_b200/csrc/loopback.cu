@@ -50,12 +50,11 @@ static int launch_ranks_inst(const GemmParams* ps_dev, int nranks, int ctas_per_
 
 int launch_ranks_kernel(int bn, int kind, int cta_group, const GemmParams* ps_dev, int nranks, int ctas_per_rank,
                         uint32_t idesc, cudaStream_t stream) {
-#define FLUXB_RANKS(BN_)                                                                                          \
-  (cta_group == 2                                                                                                  \
-       ? (kind == 0 ? launch_ranks_inst<BN_, stages_for(BN_, true), 0, true>(ps_dev, nranks, ctas_per_rank, idesc, stream)   \
-                    : launch_ranks_inst<BN_, stages_for(BN_, true), 1, true>(ps_dev, nranks, ctas_per_rank, idesc, stream))  \
-       : (kind == 0 ? launch_ranks_inst<BN_, stages_for(BN_, false), 0, false>(ps_dev, nranks, ctas_per_rank, idesc, stream) \
-                    : launch_ranks_inst<BN_, stages_for(BN_, false), 1, false>(ps_dev, nranks, ctas_per_rank, idesc, stream)))
+#define FLUXB_RANKS_KIND(BN_, CTA2_)                                                                                        \
+  (kind == 0 ? launch_ranks_inst<BN_, stages_for(BN_, CTA2_), 0, CTA2_>(ps_dev, nranks, ctas_per_rank, idesc, stream)       \
+   : kind == 1 ? launch_ranks_inst<BN_, stages_for(BN_, CTA2_), 1, CTA2_>(ps_dev, nranks, ctas_per_rank, idesc, stream)     \
+               : launch_ranks_inst<BN_, stages_for(BN_, CTA2_), 2, CTA2_>(ps_dev, nranks, ctas_per_rank, idesc, stream))
+#define FLUXB_RANKS(BN_) (cta_group == 2 ? FLUXB_RANKS_KIND(BN_, true) : FLUXB_RANKS_KIND(BN_, false))
   switch (bn) {
     case 256: return FLUXB_RANKS(256);
     case 192: return FLUXB_RANKS(192);
@@ -64,6 +63,7 @@ int launch_ranks_kernel(int bn, int kind, int cta_group, const GemmParams* ps_de
     default: FLUXB_FAIL(FLUXB_ERR_INVALID, "run_ranks: block_n=%d not in {64,128,192,256}", bn);
   }
 #undef FLUXB_RANKS
+#undef FLUXB_RANKS_KIND
 }
 
 }  // namespace fluxb

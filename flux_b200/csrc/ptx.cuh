@@ -117,6 +117,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const A
   return true;
 }
 
+// brings the cache line of `p` to L1 (small vectors read a little later) or to L2
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ----------------------------------------------------------------------------
 // proxy / scope fences
 // ----------------------------------------------------------------------------
@@ -185,6 +189,27 @@ __device__ __forceinline__ bool flag_wait_eq(const int* flag, int want, const Ab
     }
   }
   return true;
+}
+
+// The same among the CTAs of one launch (device scope): the flag is expected within about a microsecond.
+__device__ __forceinline__ bool flag_wait_eq_gpu(const int* flag, int want, const AbortWord& ab,
+                                                 int code, uint64_t budget_ns) {
+  uint64_t t0 = 0;
+  uint32_t n = 0;
+  for (;;) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    if (v == want) return true;
+    if ((++n & 15u) == 0u) {
+      if (abort_seen(ab)) return false;
+      if (t0 == 0) t0 = globaltimer_ns();
+      if (globaltimer_ns() - t0 > budget_ns) {
+        abort_raise(ab, code);
+        return false;
+      }
+      __nanosleep(32);
+    }
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -348,7 +373,7 @@ __device__ __forceinline__ uint2 ld_shared_cluster_v2(uint32_t cluster_addr) {
   return v;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_2cta(uint32_t smem_dst, uint32_t ncols) {

@@ -25,7 +25,6 @@ struct SkinnyParams {
   CUtensorMap tmap_x;  // tokens: BN rows x 128 bytes of K
   int M, N, num_kb, split;
   int w_kn;     // weight stored [K, N]
-  int acc_int;  // int8 operands
   int out_bf16, bias_mode;
   uint16_t* out;
   const uint16_t* bias;
@@ -67,7 +66,7 @@ __device__ __forceinline__ void skinny_reduce(const SkinnyParams& p, uint32_t sm
 #pragma unroll
   for (int s = 0; s < SPLIT; ++s) peer[s] = mapa_u32(smem_base + (t & 63) * 8, s);
   const float sb0 = p.scale_b != nullptr ? p.scale_b[n] : 1.0f, sb1 = p.scale_b != nullptr ? p.scale_b[n + 1] : 1.0f;
-  const bool acc_int = KIND == 1 && p.acc_int;
+  constexpr bool acc_int = KIND == 2;
   const bool has_bias = p.bias_mode != kBiasNone;
   const long long bias_pitch = p.bias_mode == kBiasFull ? p.ldbias : 0;
 #pragma unroll 1
@@ -205,7 +204,6 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyParams p, const uint32_t idesc)
       const uint64_t a_desc0 = p.w_kn ? make_mnmajor_sw128_desc(smem_base, BKE * kRowBytes) : make_kmajor_sw128_desc(smem_base);
       const uint64_t b_desc0 = make_kmajor_sw128_desc(smem_base + L::kABytes);
       const uint32_t a_step = p.w_kn ? 128u : 2u;  // 16 elements of K: 32 bytes of a K-major operand, 16 rows of an MN-major one
-      const bool acc_int = KIND == 1 && p.acc_int;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -222,7 +220,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyParams p, const uint32_t idesc)
           const uint64_t a = a_desc0 + off + a_step * k, b = b_desc0 + off + 2u * k;
           const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
           if (KIND == 0) umma_f16(tmem_base, a, b, idesc, accum);
-          else if (acc_int) umma_i8(tmem_base, a, b, idesc, accum);
+          else if (KIND == 2) umma_i8(tmem_base, a, b, idesc, accum);
           else umma_f8(tmem_base, a, b, idesc, accum);
         }
         umma_commit(bar_base + 8u * (STAGES + stage));

@@ -56,6 +56,34 @@ def test_epilogue_edges(flux, m, n, k, tuning, bias, dtype):
 
 
 @pytest.mark.parametrize("kn", [False, True])
+@pytest.mark.parametrize("m,n,bias", [(4000, 7160, "row"), (4096, 7424, "full")])
+def test_wide_tiles(flux, m, n, bias, kn):
+    """128 K blocks and three waves of 256 x 512 tiles and a cut rest: rows and columns that end inside a tile."""
+    a, b, g = _inputs(m, n, 8192, BF16)
+    t = torch.randn(1 if bias == "row" else m, n, generator=g, device="cuda").to(BF16)
+    out = flux.GemmOnly(BF16, transpose_weight=kn).forward(a, b.t().contiguous() if kn else b, bias=t)
+    _check(flux, out, a, b, t)
+
+
+def test_wide_tiles_int8(flux):
+    m, n, k = 4000, 7424, 16384
+    g = torch.Generator(device="cuda").manual_seed(9)
+    a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    one_m, one_n = torch.ones(m, device="cuda"), torch.ones(n, device="cuda")
+    out = flux.GemmOnly(torch.int8).forward(a, b, input_scale=one_m, weight_scale=one_n)
+    torch.cuda.synchronize()
+    assert torch.equal(out, (a.double() @ b.double().t()).float().to(BF16))
+
+
+def test_tile_widths_a_caller_may_not_choose(flux):
+    a, b, _ = _inputs(512, 512, 256, BF16)
+    for width in (96, 512):
+        with pytest.raises(Exception):
+            flux.GemmOnly(BF16).forward(a, b, tuning={"block_n": width})
+
+
+@pytest.mark.parametrize("kn", [False, True])
 @pytest.mark.parametrize("m", [1, 2, 16, 17, 32, 33, 64, 65, 128, 129, 256])
 @pytest.mark.parametrize("n,k", [(8, 64), (136, 264), (1160, 4096), (5000, 1032)])  # cut along K into 1, 1, 8 or 4, 4 or 2 parts
 def test_few_rows(flux, m, n, k, kn):
