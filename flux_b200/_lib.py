@@ -118,6 +118,7 @@ SIGNATURES = {
     "fluxb_moe_gather_rs_reset": (_i, [_vp, _vp]),
     "fluxb_moe_gather_rs_forward": (_i, [_vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _tun, _vp]),
     "fluxb_moe_gather_rs_set_ep": (_i, [_vp, _i, _i]),
+    "fluxb_moe_gather_rs_forward_dev": (_i, [_vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _tun, _vp]),
     "fluxb_moe_gather_rs_forward_ep": (_i, [_vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _tun, _vp]),
 }
 

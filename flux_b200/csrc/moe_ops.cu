@@ -200,6 +200,16 @@ moe_local_tables_kernel(const int* __restrict__ splits, const int* __restrict__ 
   write_tile_table(e < nexperts ? splits[e] : 0, total_rows, max_tiles, tile_m, t, status);
 }
 
+// The table alone, from splits on the device.
+__global__ void __launch_bounds__(1024)
+moe_device_tables_kernel(const int* __restrict__ splits, int nexperts, int total_rows, int max_tiles, int tile_m, MoeTables t,
+                         int* status) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_trigger();
+  const int e = threadIdx.x;
+  write_tile_table(e < nexperts ? splits[e] : 0, total_rows, max_tiles, tile_m, t, status);
+}
+
 // The same table from splits the host knows, passed by value.
 struct HostSplits {
   int v[1024];
@@ -331,6 +341,11 @@ struct fluxb_moe_gather_rs {
   unsigned long long calls;
   int ep_rank = 0, ep_size = 1;
 };
+
+static int gather_rs_forward(fluxb_moe_gather_rs* op, const void* x, int m, int ntokens, int k_local, const void* weights,
+                             const int* splits_host, const int* splits_dev, const int* routing_idx_dev, const float* in_scale,
+                             const float* w_scale, const float* vec_scale, void* out, const fluxb_tuning* tuning,
+                             fluxb_stream_t stream_);
 
 static int flag_stride_of(int full_m, int world) {
   const int per_rank = (full_m + world - 1) / world;
@@ -702,9 +717,31 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
                                    const void* weights, const int* splits_host,
                                    const int* routing_idx_dev, const float* in_scale,
                                    const float* w_scale, const float* vec_scale, void* out,
-                                   const fluxb_tuning* tuning, fluxb_stream_t stream_) {
-  FLUXB_REQUIRE(op != nullptr && x != nullptr && weights != nullptr && splits_host != nullptr &&
-                    routing_idx_dev != nullptr && out != nullptr, "moe_gather_rs_forward: NULL argument");
+                                   const fluxb_tuning* tuning, fluxb_stream_t stream) {
+  FLUXB_REQUIRE(splits_host != nullptr, "moe_gather_rs_forward: NULL argument");
+  return gather_rs_forward(op, x, m, ntokens, k_local, weights, splits_host, nullptr, routing_idx_dev, in_scale, w_scale,
+                           vec_scale, out, tuning, stream);
+}
+
+int fluxb_moe_gather_rs_forward_dev(fluxb_moe_gather_rs_t op, const void* x, int m, int k_local, const void* weights,
+                                    const int* splits_dev, const int* routing_idx_dev, const float* in_scale,
+                                    const float* w_scale, const float* vec_scale, void* out, const fluxb_tuning* tuning,
+                                    fluxb_stream_t stream) {
+  FLUXB_REQUIRE(op != nullptr && splits_dev != nullptr, "moe_gather_rs_forward_dev: NULL argument");
+  FLUXB_REQUIRE(op->comm->world == 1 && op->comm->ranks_on_gpu <= 1, "moe_gather_rs_forward_dev: needs a world-1 communicator");
+  return gather_rs_forward(op, x, m, m / op->topk, k_local, weights, nullptr, splits_dev, routing_idx_dev, in_scale, w_scale,
+                           vec_scale, out, tuning, stream);
+}
+
+}  // extern "C"
+
+// Exactly one of splits_host and splits_dev (one rank only) is given.
+static int gather_rs_forward(fluxb_moe_gather_rs* op, const void* x, int m, int ntokens, int k_local, const void* weights,
+                             const int* splits_host, const int* splits_dev, const int* routing_idx_dev, const float* in_scale,
+                             const float* w_scale, const float* vec_scale, void* out, const fluxb_tuning* tuning,
+                             fluxb_stream_t stream_) {
+  FLUXB_REQUIRE(op != nullptr && x != nullptr && weights != nullptr && routing_idx_dev != nullptr && out != nullptr,
+                "moe_gather_rs_forward: NULL argument");
   fluxb_comm* comm = op->comm;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int world = comm->world;
@@ -732,7 +769,7 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
   const int tile_m = cg == 2 ? 2 * kBM : kBM;
   std::vector<GroupTile> tiles;
   long long off = 0, row_lo = 0;
-  for (int e = 0; e < op->nexperts; ++e) {
+  for (int e = 0; splits_host != nullptr && e < op->nexperts; ++e) {
     const int cnt = splits_host[e];
     FLUXB_REQUIRE(cnt >= 0, "moe_gather_rs_forward: splits[%d]=%d is negative", e, cnt);
     if (e == e_first) row_lo = off;
@@ -750,15 +787,20 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
       FLUXB_REQUIRE(off - row_lo == m, "moe_gather_rs_forward: the splits of this rank's experts sum to %lld, expected m=%d",
                     off - row_lo, m);
   }
-  FLUXB_REQUIRE(off == rows_all, "moe_gather_rs_forward: splits sum to %lld, expected ntokens*topk=%lld", off, rows_all);
+  FLUXB_REQUIRE(splits_host == nullptr || off == rows_all, "moe_gather_rs_forward: splits sum to %lld, expected ntokens*topk=%lld", off, rows_all);
   uint8_t* ws = static_cast<uint8_t*>(op->workspace);
   void* inter = ws;
   MoeTables tb = carve_tables(ws + align_up(static_cast<size_t>(op->max_m) * n * 2, 256), op->max_m, op->nexperts);
-  const int num_tiles = static_cast<int>(tiles.size());
+  // (splits on the device: as many tiles as there can be)
+  const int num_tiles = splits_host != nullptr ? static_cast<int>(tiles.size()) : (m + tile_m - 1) / tile_m + imin(op->nexperts, m);
   // one rank: the table comes from a kernel that gets the splits by value, the GEMM only stores its rows, and the combine
   // is a launch of its own
   const bool local = world == 1 && comm->ranks_on_gpu <= 1;
-  if (local) {
+  if (splits_dev != nullptr) {
+    const int rc0 = launch_pdl(moe_device_tables_kernel, 1, 1024, stream, splits_dev, op->nexperts, static_cast<int>(rows_all),
+                               num_tiles, tile_m, tb, comm->status_dev);
+    if (rc0 != FLUXB_OK) return rc0;
+  } else if (local) {
     HostSplits hs;
     memcpy(hs.v, splits_host, static_cast<size_t>(op->nexperts) * sizeof(int));
     memset(hs.v + op->nexperts, 0, (1024 - static_cast<size_t>(op->nexperts)) * sizeof(int));
@@ -869,8 +911,6 @@ int fluxb_moe_gather_rs_forward_ep(fluxb_moe_gather_rs_t op, const void* x, int 
   op->calls += 1;
   return FLUXB_OK;
 }
-
-}  // extern "C"
 
 // ---------------------------------------------------------------------------
 // Scatter + grouped GEMM without any allocation: the routing tables live in a

@@ -216,10 +216,6 @@ def _scatter_index(chosen, nexperts):
     return _moe.calc_scatter_index(chosen, splits, return_splits=True)
 
 
-def _gather_index(scatter_index):
-    return _moe.calc_gather_index(scatter_index)
-
-
 def _make_moe_l0(group, max_tokens, hidden, ffn_hidden, nexperts, topk, dtype):
     env = _ops.DistEnvTPWithEP(group, 1, None)
     return _moe.GemmGroupedV3AGScatter(env, _ops.MoeArguments(max_tokens, hidden, ffn_hidden, nexperts, topk, dtype))
@@ -241,7 +237,7 @@ class MoEMLP(torch.nn.Module):
 
       1. router: logits of this rank's tokens, top-k with softmax weights over the chosen experts; the choices
          and weights of all ranks are all-gathered (T x topk numbers) because the routing is global;
-      2. `calc_scatter_index` / `calc_gather_index` give each (token, k) pair its row in expert order;
+      2. `calc_scatter_index` gives each (token, k) pair its row in expert order;
       3. layer 0: all-gather of the tokens + scatter + grouped GEMM in one kernel (`GemmGroupedV3AGScatter`);
       4. activation; with `gated=True` (SwiGLU-style) a second up projection `w_gate` runs over the same gathered
          tokens (`forward_multiple_weights`: the all-gather happens once) and the activation is
@@ -303,14 +299,16 @@ class MoEMLP(torch.nn.Module):
                                     self.w_up.dtype)
         chosen, weights = self.route(x_shard)
         scatter_index, splits = _scatter_index(chosen, self.nexperts)
-        gather_index, topk_index = _gather_index(scatter_index)
         # routing weight of every expert-sorted row
-        row_scale = weights.reshape(-1)[gather_index.long() * self.topk + topk_index.long()].contiguous()
+        row_scale = torch.empty_like(weights).view(-1).scatter_(0, scatter_index.view(-1).long(), weights.view(-1))
         if self.w_gate is None:
             act = self.activation(self._l0.forward(x_shard.contiguous(), self.w_up, splits, scatter_index))
         else:
             gate, up = self._l0.forward_multiple_weights(x_shard.contiguous(), [self.w_gate, self.w_up], splits,
                                                          scatter_index)
             act = self.activation(gate) * up
+        if self.world == 1 and hasattr(self._l1, "_forward"):
+            # the counts stay on the device: reading them back would hold the host until layer 0 has run
+            return self._l1._forward(act, self.w_down, None, splits, scatter_index.reshape(-1), output_vec_scale=row_scale)
         return self._l1.forward_gather_rs(act, self.w_down, splits.cpu(), scatter_index.reshape(-1),
                                           output_vec_scale=row_scale)

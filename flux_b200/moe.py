@@ -37,7 +37,7 @@ def calc_scatter_index(choosed_experts: torch.Tensor, splits: Optional[torch.Ten
         nexperts = int(choosed_experts.max().item()) + 1 if choosed_experts.numel() else 1
     chosen = choosed_experts.contiguous()
     out = torch.empty_like(chosen)
-    counts = torch.empty(nexperts, dtype=torch.int32, device=chosen.device)
+    counts = chosen.new_empty(nexperts)
     _lib.check(_lib.load().fluxb_moe_scatter_index(chosen.data_ptr(), ntokens, topk, nexperts, counts.data_ptr(),
                                                    out.data_ptr(), _cur_stream()))
     return (out, counts) if return_splits else out
@@ -50,8 +50,7 @@ def calc_gather_index(scatter_index: torch.Tensor):
            "calc_gather_index: scatter_index must be a CUDA int32 [ntokens, topk] tensor")
     ntokens, topk = scatter_index.shape
     si = scatter_index.contiguous()
-    gi = torch.empty(ntokens * topk, dtype=torch.int32, device=si.device)
-    ti = torch.empty(ntokens * topk, dtype=torch.int32, device=si.device)
+    gi, ti = si.new_empty(ntokens * topk), si.new_empty(ntokens * topk)
     _lib.check(_lib.load().fluxb_moe_gather_index(si.data_ptr(), ntokens, topk, gi.data_ptr(), ti.data_ptr(),
                                                   _cur_stream()))
     return gi, ti
@@ -107,20 +106,20 @@ class GemmGroupedV3AGScatter:
         # shape rules of src/moe_ag_scatter/ths_op/gemm_grouped_v3_ag_scatter.cc:239-265
         _check(weights.is_cuda and weights.dim() == 3 and weights.is_contiguous(), "weights must be a contiguous CUDA [E, ffn/TP, hidden] tensor")
         _check(weights.dtype == self.input_dtype, "weights dtype mismatch")
-        _check(tuple(weights.shape) == (self.nexperts_local, self.ffn_local, a.hidden),
-               f"weights shape {tuple(weights.shape)} != {(self.nexperts_local, self.ffn_local, a.hidden)}")
+        if not (tuple(weights.shape) == (self.nexperts_local, self.ffn_local, a.hidden)):
+            raise RuntimeError(f"weights shape {tuple(weights.shape)} != {(self.nexperts_local, self.ffn_local, a.hidden)}")
         _check(splits_gpu.is_cuda and splits_gpu.dtype == torch.int32 and splits_gpu.numel() >= a.nexperts,
                "splits_gpu must be a CUDA int32 tensor with at least nexperts entries")
         _check(scatter_index.is_cuda and scatter_index.dtype == torch.int32 and scatter_index.dim() == 2
                and scatter_index.shape[1] == a.topk and scatter_index.is_contiguous(),
                "scatter_index must be a contiguous CUDA int32 [ntokens, topk] tensor")
         ntokens = scatter_index.shape[0]
-        _check(ntokens % w == 0 and ntokens <= a.max_ntokens, f"ntokens={ntokens} must divide by TP and be <= max_ntokens")
+        if not (ntokens % w == 0 and ntokens <= a.max_ntokens):
+            raise RuntimeError(f"ntokens={ntokens} must divide by TP and be <= max_ntokens")
         nlocal = ntokens // w
         if not reuse:
-            _check(inputs_shard.is_cuda and inputs_shard.is_contiguous() and inputs_shard.dtype == self.input_dtype
-                   and tuple(inputs_shard.shape) == (nlocal, a.hidden),
-                   f"inputs_shard must be a contiguous [{nlocal}, {a.hidden}] tensor")
+            if not (inputs_shard.is_cuda and inputs_shard.is_contiguous() and inputs_shard.dtype == self.input_dtype and tuple(inputs_shard.shape) == (nlocal, a.hidden)):
+                raise RuntimeError(f"inputs_shard must be a contiguous [{nlocal}, {a.hidden}] tensor")
         if output_scale is not None:
             _check(output_scale.dtype == torch.float32 and output_scale.numel() == self.nexperts_local
                    and output_scale.is_contiguous(), "output_scale must be a float32 tensor with one entry per local expert")
@@ -135,7 +134,7 @@ class GemmGroupedV3AGScatter:
                 e0 = self.ep_rank * self.nexperts_local
                 rows = int(splits_gpu[e0:e0 + self.nexperts_local].sum().item())
         if outputs_buf is None:
-            outputs_buf = torch.empty((rows, self.ffn_local), dtype=self.output_dtype, device=weights.device)
+            outputs_buf = weights.new_empty((rows, self.ffn_local), dtype=self.output_dtype)
         else:
             _check(outputs_buf.dtype == self.output_dtype and outputs_buf.is_contiguous() and outputs_buf.shape[0] >= rows
                    and outputs_buf.dim() == 2 and outputs_buf.shape[1] == self.ffn_local,
@@ -208,9 +207,9 @@ class GemmGroupedV3GatherRS:
         self.ep_size = int(ep_world_size)
         self.ep_rank = int(rank) // int(tp_world_size)  # ranks of one ffn-TP group are consecutive
         self.comm = default_comm()
-        _check(self.comm.rank == int(rank) and self.comm.world == int(world_size),
-               f"GemmGroupedV3GatherRS: rank/world_size ({rank}/{world_size}) do not match the communicator of "
-               f"init_flux_shm ({self.comm.rank}/{self.comm.world})")
+        if not (self.comm.rank == int(rank) and self.comm.world == int(world_size)):
+            raise RuntimeError(f"GemmGroupedV3GatherRS: rank/world_size ({rank}/{world_size}) do not match the communicator of "
+                               f"init_flux_shm ({self.comm.rank}/{self.comm.world})")
         self.nexperts, self.max_m, self.n_dim, self.topk = int(total_num_experts), int(max_m), int(n_dim), int(topk)
         self.max_input_groups = int(max_input_groups)
         self.input_dtype = input_dtype
@@ -240,6 +239,12 @@ class GemmGroupedV3GatherRS:
     def forward_gather_rs(self, input, weight, splits_cpu, routing_idx=None, n_tokens_per_rank=None, input_scale=None,
                           weight_scale=None, output_vec_scale=None, fast_accum=False, sm_margin=0,
                           with_stream_sync=False, scatter_idx=None, tuning=None):
+        return self._forward(input, weight, splits_cpu, None, routing_idx, input_scale, weight_scale, output_vec_scale,
+                             with_stream_sync, scatter_idx, tuning)
+
+    def _forward(self, input, weight, splits_cpu, splits_gpu, routing_idx, input_scale=None, weight_scale=None,
+                 output_vec_scale=None, with_stream_sync=False, scatter_idx=None, tuning=None):
+        w = self.comm.world
         if routing_idx is None:
             routing_idx = scatter_idx  # keyword used by examples/moe.py:204-209
         _check(routing_idx is not None, "forward_gather_rs: routing_idx is required")
@@ -250,31 +255,43 @@ class GemmGroupedV3GatherRS:
                "weight must be a contiguous CUDA [E, N, K] tensor of the op's dtype")
         m, k = input.shape
         e_local = self.nexperts // self.ep_size
-        _check(tuple(weight.shape) == (e_local, self.n_dim, k), f"weight shape {tuple(weight.shape)} != {(e_local, self.n_dim, k)}")
-        _check(not splits_cpu.is_cuda and splits_cpu.dtype == torch.int32 and splits_cpu.numel() >= self.nexperts,
-               "splits_cpu must be a CPU int32 tensor with at least nexperts entries")
-        # the reference's extra splits[E] slot counts dropped tokens (gemm_grouped_v3_gather_rs.cc:668-674)
-        _check(splits_cpu.numel() == self.nexperts or int(splits_cpu[self.nexperts:].sum()) == 0,
-               "forward_gather_rs: token dropping (a non-zero splits[E] slot) is not built")
+        if not (tuple(weight.shape) == (e_local, self.n_dim, k)):
+            raise RuntimeError(f"weight shape {tuple(weight.shape)} != {(e_local, self.n_dim, k)}")
+        if splits_cpu is None:
+            # one rank, internal to the library's own layers: the tile table is made from the routing kernel's counts on the device
+            _check(w == 1 and splits_gpu.is_cuda and splits_gpu.dtype == torch.int32 and splits_gpu.numel() == self.nexperts,
+                   "splits_gpu must be a CUDA int32 tensor with nexperts entries, on one rank")
+        else:
+            _check(not splits_cpu.is_cuda and splits_cpu.dtype == torch.int32 and splits_cpu.numel() >= self.nexperts,
+                   "splits_cpu must be a CPU int32 tensor with at least nexperts entries")
+            # the reference's extra splits[E] slot counts dropped tokens (gemm_grouped_v3_gather_rs.cc:668-674)
+            _check(splits_cpu.numel() == self.nexperts or int(splits_cpu[self.nexperts:].sum()) == 0,
+                   "forward_gather_rs: token dropping (a non-zero splits[E] slot) is not built")
         _check(routing_idx.is_cuda and routing_idx.dtype == torch.int32, "routing_idx must be a CUDA int32 tensor")
         rows_all = routing_idx.numel()  # ntokens * topk; with expert parallelism `input` holds this rank's experts' rows
-        _check(rows_all % self.topk == 0 and rows_all <= self.max_m and (self.ep_size > 1 or rows_all == m),
-               f"routing_idx has {rows_all} entries for M={m} rows (max_m={self.max_m}, topk={self.topk})")
-        w = self.comm.world
+        if not (rows_all % self.topk == 0 and rows_all <= self.max_m and (self.ep_size > 1 or rows_all == m)):
+            raise RuntimeError(f"routing_idx has {rows_all} entries for M={m} rows (max_m={self.max_m}, topk={self.topk})")
         for name, s, numel in (("input_scale", input_scale, 1), ("weight_scale", weight_scale, e_local),
                                ("output_vec_scale", output_vec_scale, m)):
             if s is not None:
-                _check(s.is_cuda and s.dtype == torch.float32 and s.numel() == numel and s.is_contiguous(),
-                       f"{name} must be a contiguous CUDA float32 tensor with {numel} element(s)")
+                if not (s.is_cuda and s.dtype == torch.float32 and s.numel() == numel and s.is_contiguous()):
+                    raise RuntimeError(f"{name} must be a contiguous CUDA float32 tensor with {numel} element(s)")
         ntokens = rows_all // self.topk
-        out = torch.empty((ntokens // w, self.n_dim), dtype=self.output_dtype, device=input.device)
-        splits = splits_cpu.contiguous()
+        out = input.new_empty((ntokens // w, self.n_dim), dtype=self.output_dtype)
         if tuning is None and _tune.TABLE.records:
             tuning = _tune.TABLE.get(_tune.record_key("moe_gather_rs", m, self.n_dim, k, self.input_dtype, w))
-        _lib.check(_lib.load().fluxb_moe_gather_rs_forward_ep(
-            self._h, input.data_ptr(), m, ntokens, k, weight.data_ptr(), splits.data_ptr(),
-            routing_idx.contiguous().data_ptr(), _ptr(input_scale), _ptr(weight_scale), _ptr(output_vec_scale),
-            out.data_ptr(), _tuning(tuning), _cur_stream()))
+        lib = _lib.load()
+        if splits_cpu is None:
+            _lib.check(lib.fluxb_moe_gather_rs_forward_dev(
+                self._h, input.data_ptr(), m, k, weight.data_ptr(), splits_gpu.contiguous().data_ptr(),
+                routing_idx.contiguous().data_ptr(), _ptr(input_scale), _ptr(weight_scale), _ptr(output_vec_scale),
+                out.data_ptr(), _tuning(tuning), _cur_stream()))
+        else:
+            splits = splits_cpu.contiguous()
+            _lib.check(lib.fluxb_moe_gather_rs_forward_ep(
+                self._h, input.data_ptr(), m, ntokens, k, weight.data_ptr(), splits.data_ptr(),
+                routing_idx.contiguous().data_ptr(), _ptr(input_scale), _ptr(weight_scale), _ptr(output_vec_scale),
+                out.data_ptr(), _tuning(tuning), _cur_stream()))
         if with_stream_sync:
             torch.cuda.current_stream().synchronize()
         return out

@@ -281,6 +281,14 @@ int fluxb_moe_gather_rs_forward(fluxb_moe_gather_rs_t op, const void* x, int m, 
                                 const int* routing_idx_dev, const float* in_scale,
                                 const float* w_scale, const float* vec_scale, void* out,
                                 const fluxb_tuning* tuning, fluxb_stream_t stream);
+/* One rank: the same with the splits on the device ([nexperts] int32), so that a caller who has them there (the output
+ * of fluxb_moe_scatter_index) need not wait for the GPU. Splits that do not sum to m set the status word and leave `out`
+ * undefined. */
+int fluxb_moe_gather_rs_forward_dev(fluxb_moe_gather_rs_t op, const void* x, int m, int k_local,
+                                    const void* weights, const int* splits_dev,
+                                    const int* routing_idx_dev, const float* in_scale,
+                                    const float* w_scale, const float* vec_scale, void* out,
+                                    const fluxb_tuning* tuning, fluxb_stream_t stream);
 /* Expert parallelism (see fluxb_moe_ag_scatter_set_ep): `x` [m, k_local] and `vec_scale` [m] hold only the rows
  * of this rank's experts (m = sum of their splits), `weights` is [nexperts / ep_size, n, k_local], `splits_host`
  * and `routing_idx_dev` stay global ([nexperts] and [ntokens * topk]); every rank pushes its share of every
