@@ -224,62 +224,82 @@ moe_host_tables_kernel(const __grid_constant__ HostSplits splits, int nexperts, 
 }
 
 // out[t] = sum over k of d[scatter_index[t, k]], in fp32 in the order of k, rounded once: the combine of MoE layer 1 on
-// one rank. One thread = 8 columns of 4 tokens, so that up to 8 16-byte loads are in flight in each of 2048 threads
-// per SM. (Inside the GEMM's launch, 128 threads per SM summed column group by column group: 86 of the 443 us of 16384
-// rows x 4096 were left to do when the GEMM had ended, 117 of 243 with 8000 rows x 8192.)
-__global__ void __launch_bounds__(256)
+// one rank. One thread = 8 columns of TOK tokens; the loads of KS choices of all of them are in flight together, in 64
+// registers, so that an SM keeps 1024 threads with 8 16-byte loads each: what counts against HBM's latency. (A first
+// form, 4 tokens with their sums held over rounds of two choices, had room for 512 threads: 36.6 us for 8000 rows x 8192
+// against 27.4 here; inside the GEMM's launch, 128 threads per SM left 117 of 243 us to do after the GEMM.)
+template <int TOK, int KS, bool ONE_ROUND>
+__global__ void __launch_bounds__(256, 4)
 moe_combine_kernel(const uint16_t* __restrict__ d, const int* __restrict__ scatter_index, uint16_t* __restrict__ out,
                    int ntokens, int topk, int n, int rows, int is_bf16) {
   pdl_wait();
   if (threadIdx.x == 0) pdl_trigger();
   const int col = (static_cast<int>(blockIdx.y) * 64 + (static_cast<int>(threadIdx.x) & 63)) * 8;
-  const int t0 = (static_cast<int>(blockIdx.x) * 4 + (static_cast<int>(threadIdx.x) >> 6)) * 4;
+  const int t0 = (static_cast<int>(blockIdx.x) * 4 + (static_cast<int>(threadIdx.x) >> 6)) * TOK;
   if (col >= n) return;
-  float acc[4][8];
+  float acc[ONE_ROUND ? 1 : TOK][8];
+  if (!ONE_ROUND) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < TOK; ++j)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-  for (int k0 = 0; k0 < topk; k0 += 2) {
-    uint4 v[2][4];
+      for (int i = 0; i < 8; ++i) acc[ONE_ROUND ? 0 : j][i] = 0.f;
+  }
+  for (int k0 = 0; k0 < (ONE_ROUND ? 1 : topk); k0 += KS) {
+    uint4 v[TOK][KS];
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int j = 0; j < TOK; ++j)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[u][j] = make_uint4(0u, 0u, 0u, 0u);
-        if (k0 + u < topk && t0 + j < ntokens) {
-          const int row = scatter_index[static_cast<long long>(t0 + j) * topk + k0 + u];
-          if (row >= 0 && row < rows)  // a corrupt entry must not become a wild load
-            v[u][j] = __ldg(reinterpret_cast<const uint4*>(d + static_cast<long long>(row) * n + col));
-        }
+      for (int u = 0; u < KS; ++u) {
+        int row = -1;
+        if (t0 + j < ntokens && k0 + u < topk) row = __ldg(scatter_index + static_cast<long long>(t0 + j) * topk + k0 + u);
+        v[j][u] = make_uint4(0u, 0u, 0u, 0u);
+        if (row >= 0 && row < rows)  // a corrupt entry must not become a wild load
+          v[j][u] = __ldg(reinterpret_cast<const uint4*>(d + static_cast<long long>(row) * n + col));
       }
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int j = 0; j < TOK; ++j) {
+      float (&sum)[8] = acc[ONE_ROUND ? 0 : j];
+      if (ONE_ROUND) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t w[4] = {v[u][j].x, v[u][j].y, v[u][j].z, v[u][j].w};
+        for (int i = 0; i < 8; ++i) sum[i] = 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < KS; ++u) {
+        const uint32_t w[4] = {v[j][u].x, v[j][u].y, v[j][u].z, v[j][u].w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          if (is_bf16) {
-            acc[j][2 * i] += __uint_as_float(w[i] << 16);
-            acc[j][2 * i + 1] += __uint_as_float(w[i] & 0xFFFF0000u);
-          } else {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            acc[j][2 * i] += f.x;
-            acc[j][2 * i + 1] += f.y;
-          }
+          const float2 f = is_bf16 ? make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u))
+                                   : __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+          sum[2 * i] += f.x;
+          sum[2 * i + 1] += f.y;
         }
       }
-  }
+      if ((ONE_ROUND || k0 + KS >= topk) && t0 + j < ntokens) {
+        uint32_t w[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (t0 + j < ntokens) {
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        w[i] = is_bf16 ? pack_bf16(acc[j][2 * i], acc[j][2 * i + 1]) : pack_f16(acc[j][2 * i], acc[j][2 * i + 1]);
-      *reinterpret_cast<uint4*>(out + static_cast<long long>(t0 + j) * n + col) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int i = 0; i < 4; ++i) w[i] = is_bf16 ? pack_bf16(sum[2 * i], sum[2 * i + 1]) : pack_f16(sum[2 * i], sum[2 * i + 1]);
+        *reinterpret_cast<uint4*>(out + static_cast<long long>(t0 + j) * n + col) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
+  }
+}
+
+template <int TOK, int KS, bool ONE_ROUND>
+static int launch_combine(const void* d, const int* scatter_index, void* out, int ntokens, int topk, int n, int rows, bool is_bf16,
+                          cudaStream_t stream) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(static_cast<unsigned>((ntokens + 4 * TOK - 1) / (4 * TOK)), static_cast<unsigned>((n / 8 + 63) / 64), 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  FLUXB_CUDA(cudaLaunchKernelEx(&cfg, moe_combine_kernel<TOK, KS, ONE_ROUND>, static_cast<const uint16_t*>(d), scatter_index,
+                                static_cast<uint16_t*>(out), ntokens, topk, n, rows, is_bf16 ? 1 : 0));
+  return FLUXB_OK;
 }
 
 // Visiting order of the tiles: stable counting sort by how late the tile's last source block is permuted
@@ -840,25 +860,17 @@ static int gather_rs_forward(fluxb_moe_gather_rs* op, const void* x, int m, int 
   if (rc != FLUXB_OK) return rc;
   encode_out_map(p, inter, p.M, n, p.out_type);
   if (local) {
+    p.epi_wide = 1;
     fluxb_tuning tl = tuning != nullptr ? *tuning : fluxb_tuning{0, 0, 0, 0, 0};
     tl.block_n = bn;
     tl.cta_group = cg;
     rc = launch_fused_gemm(comm, p, op->in_dtype, &tl, stream);
     if (rc != FLUXB_OK) return rc;
     op->calls += 1;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(static_cast<unsigned>((ntokens + 15) / 16), static_cast<unsigned>((n / 8 + 63) / 64), 1);
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FLUXB_CUDA(cudaLaunchKernelEx(&cfg, moe_combine_kernel, static_cast<const uint16_t*>(inter), routing_idx_dev,
-                                  static_cast<uint16_t*>(out), ntokens, topk, n, m, op->out_dtype == FLUXB_BF16 ? 1 : 0));
-    return FLUXB_OK;
+    const bool bf16 = op->out_dtype == FLUXB_BF16;
+    if (topk <= 2) return launch_combine<4, 2, true>(inter, routing_idx_dev, out, ntokens, topk, n, m, bf16, stream);
+    if (topk <= 4) return launch_combine<2, 4, true>(inter, routing_idx_dev, out, ntokens, topk, n, m, bf16, stream);
+    return launch_combine<2, 4, false>(inter, routing_idx_dev, out, ntokens, topk, n, m, bf16, stream);
   }
   // combine + reduce-scatter run inside the same launch (comm warps), column slab by column slab
   const int parity = static_cast<int>(op->calls & 1ull);
