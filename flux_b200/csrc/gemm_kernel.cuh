@@ -481,8 +481,9 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     }
   }
   tc_fence_before();
-  // A dense plain GEMM touches global memory first with its producer's loads, which wait there; every other mode reads
-  // tables, counters or tokens in several roles.
+  // A dense plain GEMM touches global memory first with its producer's loads, and waits there; every other mode reads
+  // tables, counters or tokens in several roles. The roles that follow the producer wait as well: the budget of their
+  // first bounded wait must not run while the kernel before this one still does.
   const bool pdl_late = p.g_tiles == nullptr && p.epi_mode == kEpiStore && p.ag_flags == nullptr && p.ag_src == nullptr;
   if (!pdl_late) pdl_wait();
   if (CTA2) cluster_sync_all(); else __syncthreads();
@@ -857,6 +858,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       const uint64_t a_desc0 = make_kmajor_sw128_desc(smem_a(0));
       const uint64_t b_desc0 = b_kn ? make_mnmajor_sw128_desc(smem_b(0), BKE * kRowBytes) : make_kmajor_sw128_desc(smem_b(0));
       const uint32_t b_step = b_kn ? 128u : 2u;
+      if (pdl_late) pdl_wait();
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -915,6 +917,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
     }
   } else if (warp < 6 || (p.epi_wide && L::kEpiBufs == 2)) {
     // ------------------------------------------------------------- epilogue
+    if (pdl_late) pdl_wait();
     const bool wide = p.epi_wide && L::kEpiBufs == 2;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;

@@ -222,6 +222,7 @@ plain_gemm_kernel(const __grid_constant__ PlainParams p, const uint32_t idesc) {
       const uint64_t b_desc0 = b_kn ? make_mnmajor_sw128_desc(smem_base + L::kABytes, BKE * kRowBytes)
                                     : make_kmajor_sw128_desc(smem_base + L::kABytes);
       const uint32_t b_step = b_kn ? 128u : 2u;
+      pdl_wait();  // (the budget of the waits below starts when the kernel before this one has ended)
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;

@@ -204,6 +204,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyParams p, const uint32_t idesc)
       const uint64_t a_desc0 = p.w_kn ? make_mnmajor_sw128_desc(smem_base, BKE * kRowBytes) : make_kmajor_sw128_desc(smem_base);
       const uint64_t b_desc0 = make_kmajor_sw128_desc(smem_base + L::kABytes);
       const uint32_t a_step = p.w_kn ? 128u : 2u;  // 16 elements of K: 32 bytes of a K-major operand, 16 rows of an MN-major one
+      pdl_wait();  // (the budget of the waits below starts when the kernel before this one has ended)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -244,6 +245,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyParams p, const uint32_t idesc)
     // UMMAs have retired by then, so the stages are free)
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
+    pdl_wait();  // (as above)
     if (__all_sync(0xffffffffu, mbar_wait(bar_done, 0, ab, kStatusTimeoutTmemFull, p.timeout_ns))) {
       tc_fence_after();
       const uint32_t t0 = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
