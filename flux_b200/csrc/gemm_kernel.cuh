@@ -489,7 +489,9 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
   if (CTA2) cluster_sync_all(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  if (threadIdx.x == 0) pdl_trigger();
+  // (With several ranks the next launch starts when this one has ended: its CTAs, waiting on this GPU, could take the SMs of
+  // work that a peer waits for, while this kernel waits for the peer.)
+  if (threadIdx.x == 0 && p.world == 1) pdl_trigger();
 
   const int n_tiles = (p.N + BN - 1) / BN;
   int tps = 1, m_tiles;

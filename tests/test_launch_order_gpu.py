@@ -1,6 +1,13 @@
 """Launches that may become resident while the launch before them still runs (programmatic dependent launch)."""
+import ctypes as C
+import os
+import sys
+
 import pytest
 import torch
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+from ranks_on_gpu import Ranks, _p, _stream  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 BF16 = torch.bfloat16
@@ -41,3 +48,41 @@ def test_the_wait_budget_starts_when_the_launch_before_has_ended(flux, m, bias):
     flux.get_comm(None).check_status()
     assert start.elapsed_time(end) > 30, "the first launch is meant to last several budgets"
     assert torch.equal(out, want)
+
+
+def test_nothing_starts_beside_a_launch_that_waits_for_a_peer(flux):
+    """Rank 0 of two runs alone and gives up on its peer after 300 ms; most of its CTAs have nothing to do by then.
+    A plain GEMM behind it enters the GPU only when it has ended (and is not disturbed by it)."""
+    from flux_b200 import _lib
+
+    lib, n, k, m_local = _lib.load(), 256, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(7)
+    a = torch.randn(512, k, generator=g, device="cuda").to(BF16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.02).to(BF16)
+    op = flux.GemmOnly(BF16)
+    want = op.forward(a, b)
+    comm = flux.get_comm(None)
+    comm.set_timeout_ms(100)
+    words = torch.cuda.get_device_properties(0).multi_processor_count * 8
+    first, second = (torch.zeros(words, dtype=torch.int64, device="cuda") for _ in range(2))
+    rk = Ranks(2, timeout_ms=300)
+    try:
+        ops = rk.ag_gemm_ops(2 * m_local, n, k, BF16, BF16)
+        gathered = torch.zeros(2 * m_local, n, dtype=BF16, device="cuda")
+        _lib.check(lib.fluxb_comm_set_ranks_on_gpu(rk.comms[0], 1))
+        _lib.check(lib.fluxb_comm_set_trace(rk.comms[0], _p(first)))
+        _lib.check(lib.fluxb_comm_set_trace(comm.handle, _p(second)))
+        _lib.check(lib.fluxb_ag_gemm_forward(ops[0], _p(a), m_local, _p(b), n, k, _p(gathered), None, 0, None, None, 1.0, 0, None,
+                                             None, _stream()))
+        out = op.forward(a, b)
+        torch.cuda.synchronize()
+        status = C.c_int(-1)
+        _lib.check(lib.fluxb_status_peek(rk.comms[0], C.byref(status)))
+        assert status.value == 5  # the wait for the peer's rows ran out
+        comm.check_status()
+        assert torch.equal(out, want)
+        entered = second.view(-1, 8)[:, 0]
+        assert int(entered[entered > 0].min()) >= int(first.view(-1, 8)[:, 3:5].max())
+    finally:
+        _lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
+        rk.close()
