@@ -279,6 +279,11 @@ __host__ __device__ __forceinline__ int splitk_parts(int tail_tiles, int workers
   return parts >= 2 && (scatter || num_kb - num_kb / parts >= 32) ? parts : 1;
 }
 
+// The same for launch `p` of `total_tiles` tiles: the kernel's split, and the host's question whether it needs scratch.
+__host__ __device__ __forceinline__ int tail_split(const GemmParams& p, int total_tiles, int workers, int num_kb) {
+  return p.g_tiles == nullptr ? splitk_parts(total_tiles % workers, workers, num_kb, p.epi_mode == kEpiRsPush) : 1;
+}
+
 // Split-K tail: which part finishes the 32-column step `c` of a tail tile that is BN columns wide and cut into
 // `split` parts. Steps are owned in pairs (one 64-column box = one staged store), box b by part
 // b * owners / boxes with owners = min(split, boxes); parts >= owners only park. A tile that is pushed to
@@ -514,7 +519,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
   const int full_waves = total_tiles / tile_step;
   const int full_tiles = full_waves * tile_step;
   const int tail_tiles = total_tiles - full_tiles;
-  const int split = p.splitk_scratch != nullptr && p.g_tiles == nullptr ? splitk_parts(tail_tiles, tile_step, num_kb, p.epi_mode == kEpiRsPush) : 1;
+  const int split = p.splitk_scratch != nullptr ? tail_split(p, total_tiles, tile_step, num_kb) : 1;
   auto get_item = [&](int i, int& t, int& kb0, int& kb1, int& part) -> bool {
     part = 0;
     kb0 = 0;

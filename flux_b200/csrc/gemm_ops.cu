@@ -14,8 +14,18 @@ namespace fluxb {
 // ---------------------------------------------------------------------------
 // launcher
 // ---------------------------------------------------------------------------
+template <class Params>
+static int take_splitk_slot(fluxb_comm* comm, Params& p, cudaStream_t stream) {
+  SplitkSlot s;
+  const int rc = splitk_slot(comm, stream, &s);
+  p.splitk_scratch = s.scratch;
+  p.splitk_cnt = s.cnt;
+  p.splitk_done = s.done;
+  return rc;
+}
+
 template <int BN, int STAGES, int KIND, bool CTA2>
-static int launch_inst(const fluxb_comm* comm, const GemmParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+static int launch_inst(fluxb_comm* comm, GemmParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
   // (several ranks: the launch order of kernels that wait on one another stays the stream's)
   const bool pdl = comm->world == 1;
   using L = SmemLayout<BN, STAGES, CTA2>;
@@ -55,6 +65,14 @@ static int launch_inst(const fluxb_comm* comm, const GemmParams& p, uint32_t ide
     grid &= ~1;
     if (grid > 2 * max_clusters[dev]) grid = 2 * max_clusters[dev];
     if (grid < 2) grid = 2;
+  }
+  if (p.g_tiles == nullptr) {
+    constexpr int kTileM = CTA2 ? 2 * kBM : kBM, kBlockK = kRowBytes / (KIND == 0 ? 2 : 1);
+    const int tiles = p.nseg * ((p.seg_rows + kTileM - 1) / kTileM) * ((p.N + BN - 1) / BN);
+    if (tail_split(p, tiles, CTA2 ? grid / 2 : grid, (p.K + kBlockK - 1) / kBlockK) > 1) {
+      const int rc = take_splitk_slot(comm, p, stream);
+      if (rc != FLUXB_OK) return rc;
+    }
   }
   cfg.gridDim = dim3(grid, 1, 1);
   if (pdl) cfg.numAttrs = 2;
@@ -242,9 +260,7 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
   p.status = comm->status_dev;
   p.timeout_ns = comm->timeout_ns;
   p.trace = comm->trace;
-  p.splitk_scratch = comm->splitk_scratch;
-  p.splitk_cnt = comm->splitk_cnt;
-  p.splitk_done = comm->splitk_cnt + comm->sm_count * 8;
+  p.splitk_scratch = nullptr;  // (given out by launch_inst, to launches that are cut)
   p.rank = comm->rank;
   p.world = comm->world;
   const int kind = kind_of(in_dtype);
@@ -256,6 +272,8 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
   const uint32_t idesc = make_idesc(fmt, cg == 2 ? 2 * kBM : kBM, static_cast<uint32_t>(bn), p.b_mn_major ? 1u : 0u,
                                     is_int8(in_dtype) ? 2u : 1u);
   if (comm->ranks_on_gpu > 1) {
+    const int rc = take_splitk_slot(comm, p, stream);  // (the merged launch is synchronous: no other one runs beside it)
+    if (rc != FLUXB_OK) return rc;
     DeferredItem it;
     it.fused = true;
     it.p = p;
@@ -402,7 +420,7 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
 // plain GEMM (plain_gemm.cuh)
 // ---------------------------------------------------------------------------
 template <int BN, int KIND, bool CTA2>
-static int launch_plain_inst(const fluxb_comm* comm, PlainParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+static int launch_plain_inst(fluxb_comm* comm, PlainParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
   using L = PlainLayout<BN, CTA2>;
   auto kern = plain_gemm_kernel<BN, KIND, CTA2>;
   static bool configured[64] = {};
@@ -447,6 +465,11 @@ static int launch_plain_inst(const fluxb_comm* comm, PlainParams& p, uint32_t id
   p.split = splitk_parts(p.tail_tiles, workers, p.num_kb, false);
   // the scratch holds 128 x 256 accumulators per SM: enough for any cut of tiles up to 256 columns, not of 512
   while (p.split > 1 && static_cast<long long>(p.split - 1) * p.tail_tiles * per * BN > static_cast<long long>(comm->sm_count) * 256) --p.split;
+  if (p.split > 1) {
+    const int rc = take_splitk_slot(comm, p, stream);
+    if (rc != FLUXB_OK) return rc;
+    if (p.splitk_scratch == nullptr) p.split = 1;
+  }
   p.split_div.set(static_cast<uint32_t>(p.split));
   cfg.gridDim = dim3(workers * per, 1, 1);
   cfg.numAttrs = 2;
@@ -465,7 +488,7 @@ static bool wide_tile_wins(int sm_count, int m, int n, long long row_bytes) {
 }
 
 // 16-bit output; output, bias and column scales 16-byte aligned.
-static int launch_plain(const fluxb_comm* comm, const GemmParams& g, const void* a, const void* b, int in_dtype, int bn, int cg,
+static int launch_plain(fluxb_comm* comm, const GemmParams& g, const void* a, const void* b, int in_dtype, int bn, int cg,
                         const fluxb_tuning* tuning, cudaStream_t stream) {
   FLUXB_REQUIRE(!g.b_mn_major || (bn / cg) % 64 == 0,
                 "a [K,N] weight needs a tile width whose per-CTA share is a multiple of 64 (block_n=%d, cta_group=%d)", bn, cg);
@@ -493,9 +516,6 @@ static int launch_plain(const fluxb_comm* comm, const GemmParams& g, const void*
   p.scale_b = g.scale_b;
   p.out = static_cast<uint16_t*>(g.out);
   p.bias = static_cast<const uint16_t*>(g.bias);
-  p.splitk_scratch = comm->splitk_scratch;
-  p.splitk_cnt = comm->splitk_cnt;
-  p.splitk_done = comm->splitk_cnt + comm->sm_count * 8;
   p.trace = comm->trace;
   p.status = comm->status_dev;
   p.timeout_ns = comm->timeout_ns;

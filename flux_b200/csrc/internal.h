@@ -8,6 +8,8 @@
 #include <string.h>
 
 #include <functional>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -98,6 +100,39 @@ struct DeferredItem {
   int bn = 0, kind = 0, cta_group = 1, grid = 0;
   std::function<int(cudaStream_t)> plain;
 };
+
+// Who uses which slot of the split-K scratch. A cut launch parks partial sums and counts parts in memory that no other
+// launch may touch meanwhile, so a slot belongs to one queue of launches that follow one another: a stream
+// (`capture` = 0, for the life of the communicator: stream ids are never given twice), or a stream inside one capture,
+// whose launches run again with the graph, beside anything else (until the graph is gone). A queue that comes when all
+// slots are taken gets none, and its launches are not cut: slower, never wrong.
+constexpr int kSplitkSlots = 8;
+struct SplitkOwners {
+  std::mutex mu;
+  struct Queue {
+    bool used = false;
+    unsigned long long capture = 0, stream = 0;
+  } slot[kSplitkSlots];
+  // slot of the queue, or -1; *fresh = the queue had none before
+  int claim(unsigned long long capture, unsigned long long stream, bool* fresh) {
+    std::lock_guard<std::mutex> lock(mu);
+    *fresh = false;
+    int spare = -1;
+    for (int i = kSplitkSlots - 1; i >= 0; --i) {
+      if (!slot[i].used) spare = i;
+      else if (slot[i].capture == capture && slot[i].stream == stream) return i;
+    }
+    if (spare < 0) return -1;
+    slot[spare].used = *fresh = true;
+    slot[spare].capture = capture;
+    slot[spare].stream = stream;
+    return spare;
+  }
+  void release(int i) {
+    std::lock_guard<std::mutex> lock(mu);
+    slot[i].used = false;
+  }
+};
 }  // namespace fluxb
 
 struct fluxb_comm {
@@ -110,8 +145,11 @@ struct fluxb_comm {
   unsigned long long timeout_ns = 10ull * 1000 * 1000 * 1000;
   int barrier_epoch = 0;
   unsigned long long* trace = nullptr;  // optional per-CTA timeline buffer (caller-owned device memory)
-  float* splitk_scratch = nullptr;  // sm_count x 128 x 256 fp32: parked partial accumulators of split tail tiles
-  int* splitk_cnt = nullptr;        // per (tail tile, half, epilogue warp) arrivals, zero between launches
+  // [kSplitkSlots] of: sm_count x 128 x 256 fp32 parked partial accumulators of split tail tiles, and per (tail tile, half,
+  // epilogue warp) the two counters of the parts, zero between launches
+  float* splitk_scratch = nullptr;
+  int* splitk_cnt = nullptr;
+  std::shared_ptr<fluxb::SplitkOwners> splitk_owners = std::make_shared<fluxb::SplitkOwners>();
   // several ranks on one GPU (test harness): forwards queue their stream work here, fluxb_run_ranks issues it
   int ranks_on_gpu = 1;
   std::vector<fluxb::DeferredItem> deferred;
@@ -179,6 +217,14 @@ int resolve_cta_group(const GemmParams& p, const fluxb_tuning* tuning);
 // ranks share the GPU).
 int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
                       const fluxb_tuning* tuning, cudaStream_t stream);
+
+// Scratch and counters for the cut launches of `stream`; null pointers if there is none for it (the launch is not cut then).
+struct SplitkSlot {
+  float* scratch = nullptr;
+  int* cnt = nullptr;   // parts that have parked
+  int* done = nullptr;  // parts that have seen all others parked
+};
+int splitk_slot(fluxb_comm* comm, cudaStream_t stream, SplitkSlot* out);
 
 // Run `fn(stream)` now, or queue it behind the queued launches while several ranks share the GPU.
 int enqueue_or_defer(fluxb_comm* comm, cudaStream_t stream, std::function<int(cudaStream_t)> fn);

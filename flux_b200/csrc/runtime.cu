@@ -116,6 +116,58 @@ int encode_tmap_b16_store(CUtensorMap* out, const void* base, long long rows, lo
   return FLUXB_OK;
 }
 
+static size_t splitk_slot_floats(int sms) { return static_cast<size_t>(sms) * kBM * 256; }
+static size_t splitk_slot_counters(int sms) { return static_cast<size_t>(sms) * 16; }  // "parked" and "seen"
+
+int splitk_slot(fluxb_comm* comm, cudaStream_t stream, SplitkSlot* out) {
+  *out = SplitkSlot();
+  cudaStreamCaptureStatus status;
+  unsigned long long capture = 0, id = 0;
+  cudaGraph_t graph = nullptr;
+  FLUXB_CUDA(cudaStreamGetCaptureInfo_v2(stream, &status, &capture, &graph, nullptr, nullptr));
+  if (status == cudaStreamCaptureStatusInvalidated) return FLUXB_OK;  // the launch will report it
+  if (status == cudaStreamCaptureStatusActive) {
+    id = reinterpret_cast<uintptr_t>(stream);  // (the id proper may not be asked for during a capture)
+  } else {
+    capture = 0;
+    FLUXB_CUDA(cudaStreamGetId(stream, &id));
+  }
+  bool fresh = false;
+  const int i = comm->splitk_owners->claim(capture, id, &fresh);
+  if (i < 0) return FLUXB_OK;
+  if (fresh && capture != 0) {
+    // the graph, and every executable made from it, keeps the slot; the last of them to go gives it back
+    struct Hold {
+      std::shared_ptr<SplitkOwners> owners;
+      int slot;
+    };
+    Hold* hold = new Hold{comm->splitk_owners, i};
+    cudaUserObject_t obj;
+    cudaError_t e = cudaUserObjectCreate(
+        &obj, hold,
+        [](void* h) {
+          Hold* held = static_cast<Hold*>(h);
+          held->owners->release(held->slot);
+          delete held;
+        },
+        1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+      comm->splitk_owners->release(i);
+      delete hold;
+      FLUXB_CUDA(e);
+    }
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+      cudaUserObjectRelease(obj, 1);  // runs the callback
+      FLUXB_CUDA(e);
+    }
+  }
+  out->scratch = comm->splitk_scratch + i * splitk_slot_floats(comm->sm_count);
+  out->cnt = comm->splitk_cnt + i * splitk_slot_counters(comm->sm_count);
+  out->done = out->cnt + comm->sm_count * 8;
+  return FLUXB_OK;
+}
+
 // One block, one thread per peer. Epoch-valued handshake: rank r stores the
 // epoch into slot r of every peer's array, then waits until every slot of its
 // own array has reached the epoch. Values only grow, so nothing is reset.
@@ -196,9 +248,9 @@ int fluxb_comm_create(int rank, int world, fluxb_comm_t* out) {
     delete c;
     FLUXB_FAIL(FLUXB_ERR_CUDA, "cudaHostGetDevicePointer failed: %s", cudaGetErrorString(e));
   }
-  // scratch of the split-K tail: one 128 x 256 fp32 tile per SM bounds every launch's need
-  const size_t sk_bytes = static_cast<size_t>(sms) * kBM * 256 * sizeof(float);
-  const size_t cnt_bytes = static_cast<size_t>(sms) * 16 * sizeof(int);  // "parked" and "seen" counters
+  // slots of the split-K tail: one 128 x 256 fp32 tile per SM bounds every launch's need (19.4 MB a slot on 148 SMs)
+  const size_t sk_bytes = kSplitkSlots * splitk_slot_floats(sms) * sizeof(float);
+  const size_t cnt_bytes = kSplitkSlots * splitk_slot_counters(sms) * sizeof(int);
   if (cudaMalloc(reinterpret_cast<void**>(&c->splitk_scratch), sk_bytes) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&c->splitk_cnt), cnt_bytes) != cudaSuccess ||
       cudaMemset(c->splitk_cnt, 0, cnt_bytes) != cudaSuccess) {
@@ -252,7 +304,7 @@ int fluxb_status_clear(fluxb_comm_t comm) {
     int cur = -1;
     FLUXB_CUDA(cudaGetDevice(&cur));
     if (cur != comm->device) FLUXB_CUDA(cudaSetDevice(comm->device));
-    const cudaError_t e = cudaMemset(comm->splitk_cnt, 0, static_cast<size_t>(comm->sm_count) * 16 * sizeof(int));
+    const cudaError_t e = cudaMemset(comm->splitk_cnt, 0, kSplitkSlots * splitk_slot_counters(comm->sm_count) * sizeof(int));
     if (cur != comm->device) cudaSetDevice(cur);
     FLUXB_CUDA(e);
   }

@@ -99,3 +99,16 @@ extern "C" int probe_rs_late_peers(int nseg, int seg_rows, int cta_group) {
 // Owner part of column step c of a split tail tile (splitk_owner_of / splitk_owners of gemm_kernel.cuh).
 extern "C" int probe_splitk_owner(int c, int split, int bn, int pushed) { return splitk_owner_of(c, split, bn, pushed != 0); }
 extern "C" int probe_splitk_owners(int split, int bn, int pushed) { return splitk_owners(split, bn, pushed != 0); }
+
+// Queues of launches and the split-K slots they are given (SplitkOwners of internal.h): `ops` is n triples
+// (capture, stream, slot to release first or -1); got[i] = slot, fresh[i] = whether it was new to the queue.
+extern "C" int probe_splitk_slots(const int* ops, int n, int* got, int* fresh) {
+  SplitkOwners owners;
+  for (int i = 0; i < n; ++i) {
+    if (ops[3 * i + 2] >= 0) owners.release(ops[3 * i + 2]);
+    bool f = false;
+    got[i] = owners.claim(static_cast<unsigned long long>(ops[3 * i]), static_cast<unsigned long long>(ops[3 * i + 1]), &f);
+    fresh[i] = f ? 1 : 0;
+  }
+  return kSplitkSlots;
+}

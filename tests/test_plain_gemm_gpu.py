@@ -3,6 +3,9 @@ that end inside a warp's 32 rows or a 64-column box, vectors that are not 16-byt
 
 Bound of every element: half a unit in the last place of the 16-bit output, taken twice (2^-8 of the value for bf16,
 2^-11 for fp16), plus K roundings of fp32 sums, K * 2^-23 * sum |a| |b|. int8 is compared bit for bit."""
+import ctypes as C
+import time
+
 import pytest
 import torch
 
@@ -154,3 +157,108 @@ def test_int8_accumulators_cut_along_k_stay_whole_numbers(flux, m, n, tuning):
         torch.cuda.synchronize()
         flux.get_comm(None).check_status()
         assert torch.equal(out, (a.double() @ b.double().t()).float().to(BF16))
+
+
+class _OwnComm:
+    """A communicator without any stream's scratch taken yet."""
+
+    def __init__(self):
+        from flux_b200 import _lib
+
+        self.lib, self.handle = _lib.load(), C.c_void_p()
+        _lib.check(self.lib.fluxb_comm_create(0, 1, C.byref(self.handle)))
+        _lib.check(self.lib.fluxb_comm_set_timeout_ms(self.handle, 5000))
+
+    def check_status(self):
+        torch.cuda.synchronize()
+        status = C.c_int(-1)
+        assert self.lib.fluxb_status_peek(self.handle, C.byref(status)) == 0 and status.value == 0
+
+    def __del__(self):
+        self.lib.fluxb_comm_destroy(self.handle)
+
+
+def _cut_launch(flux, dtype, num_ctas):
+    """38 tiles of 256 x 256: one is left to be cut into 8 parts on 37 CTA pairs (74 CTAs), two on 18 (36 CTAs)."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    m, n, k, tuning = 512, 19 * 256, 16384, {"block_n": 256, "cta_group": 2, "num_ctas": num_ctas}
+    if dtype == torch.int8:
+        a, a2, b = (torch.randint(-127, 128, (r, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8) for r in (m, m, n))
+        kw = {"input_scale": torch.ones(m, device="cuda"), "weight_scale": torch.ones(n, device="cuda")}
+    else:
+        a, a2, b = (torch.randn(r, k, generator=g, device="cuda").to(dtype) for r in (m, m, n))
+        kw = {}
+    op = flux.GemmOnly(dtype)
+    op.comm = _OwnComm()
+    return op.comm, a, a2, lambda x, out=None, bias=None: op.forward(x, b, output_buf=out, bias=bias, tuning=tuning, **kw)
+
+
+@pytest.mark.parametrize("kernel", ["plain", "fused"])
+@pytest.mark.parametrize("dtype", [BF16, torch.int8])
+def test_cut_launches_on_two_streams(flux, dtype, kernel):
+    """Two launches side by side on half the SMs each, each with parts of its own last wave: the results of one after the
+    other. (An unaligned bias takes the fused kernel.)"""
+    comm, a, a2, call = _cut_launch(flux, dtype, 74)
+    bias = None if kernel == "plain" else torch.ones(19 * 256 + 1, device="cuda", dtype=BF16)[1:].view(1, -1)
+    want = [call(a, bias=bias), call(a2, bias=bias)]
+    comm.check_status()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = [[], []]
+    for _ in range(20):
+        for i, x in enumerate((a, a2)):
+            with torch.cuda.stream(streams[i]):
+                outs[i].append(call(x, bias=bias))
+    comm.check_status()
+    for i in range(2):
+        assert all(torch.equal(o, want[i]) for o in outs[i])
+
+
+def test_cut_launches_in_graphs_beside_eager_ones(flux):
+    """Two graphs captured on one stream, replayed on two others beside eager launches on that stream."""
+    comm, a, a2, call = _cut_launch(flux, BF16, 36)
+    want, want2 = call(a), call(a2)
+    outs = [torch.empty_like(want) for _ in range(3)]
+    side = [torch.cuda.Stream() for _ in range(3)]
+    comm.check_status()
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+    for graph, x, out in zip(graphs, (a, a2), outs):
+        with torch.cuda.graph(graph, stream=side[2]):
+            call(x, out)
+    for _ in range(10):
+        for i in range(2):
+            with torch.cuda.stream(side[i]):
+                graphs[i].replay()
+        with torch.cuda.stream(side[2]):
+            call(a, outs[2])
+    comm.check_status()
+    assert torch.equal(outs[0], want) and torch.equal(outs[1], want2) and torch.equal(outs[2], want)
+
+
+def test_graphs_give_their_scratch_back(flux):
+    """More graphs, one after the other, than there is scratch for: the last is cut like the first (the same sums)."""
+    comm, a, _, call = _cut_launch(flux, BF16, 74)
+    want = call(a)
+    stream = torch.cuda.Stream()
+    for _ in range(12):
+        out = torch.empty_like(want)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            call(a, out)
+        graph.replay()
+        comm.check_status()
+        assert torch.equal(out, want)
+        del graph
+        time.sleep(0.1)  # the driver gives it back from a thread of its own
+
+
+def test_more_streams_than_scratch(flux):
+    """Streams that come when all scratch is taken run uncut; whole-number sums are the same."""
+    comm, a, _, call = _cut_launch(flux, torch.int8, 74)
+    want = call(a)
+    outs = []
+    for stream in [torch.cuda.Stream() for _ in range(20)]:
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            outs.append(call(a))
+    comm.check_status()
+    assert all(torch.equal(o, want) for o in outs)

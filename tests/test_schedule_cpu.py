@@ -46,6 +46,8 @@ def probe():
         fn.restype = C.c_int
     lib.probe_splitk_owner.argtypes = [C.c_int] * 4
     lib.probe_splitk_owners.argtypes = [C.c_int] * 3
+    lib.probe_splitk_slots.restype = C.c_int
+    lib.probe_splitk_slots.argtypes = [C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.probe_rs_late_peers.restype = C.c_int
     lib.probe_rs_late_peers.argtypes = [C.c_int] * 3
     lib.probe_resolve.restype = None
@@ -222,3 +224,19 @@ def test_split_tail_box_ownership(probe):
                 assert all(own[c] == own[c ^ 1] for c in range(steps))
             assert probe.probe_splitk_owners(split, bn, 1) == 1
             assert all(probe.probe_splitk_owner(c, split, bn, 1) == 0 for c in range(steps))
+
+
+def test_split_scratch_is_never_shared_by_launches_that_may_overlap(probe):
+    """Streams, and streams inside captures, each have a slot of their own and keep it; one that comes when all are taken
+    gets none, until a graph has given its slot back."""
+    nslots = probe.probe_splitk_slots((C.c_int * 1)(), 0, (C.c_int * 1)(), (C.c_int * 1)())
+    queues = [(0, 10), (0, 11), (5, 10), (5, 11), (6, 10)] + [(0, 20 + i) for i in range(nslots)]
+    ops = [(c, s, -1) for c, s in queues] + [(c, s, -1) for c, s in queues] + [(7, 10, 2), (5, 10, -1)]
+    flat = [x for op in ops for x in op]
+    got, fresh = (C.c_int * len(ops))(), (C.c_int * len(ops))()
+    probe.probe_splitk_slots((C.c_int * len(flat))(*flat), len(ops), got, fresh)
+    n = len(queues)
+    assert list(got[:nslots]) == list(range(nslots)) and all(fresh[:nslots])
+    assert all(g == -1 for g in got[nslots:n]) and list(got[:n]) == list(got[n:2 * n]) and not any(fresh[nslots:2 * n])
+    assert got[2 * n] == 2 and fresh[2 * n] == 1  # the slot that queue (5, 10) gave back
+    assert got[2 * n + 1] == -1
