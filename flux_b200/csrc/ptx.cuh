@@ -372,8 +372,10 @@ __device__ __forceinline__ uint2 ld_shared_cluster_v2(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(cluster_addr) : "memory");
   return v;
 }
+// Arrival at a barrier of another CTA of the cluster. The default scope is the CTA, which does not order the arriving
+// warps' reads of tensor memory before what the other CTA issues once it has seen them.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_2cta(uint32_t smem_dst, uint32_t ncols) {

@@ -102,3 +102,16 @@ def test_gemm_only_rejects_unsupported_modes():
         flux.GemmOnly(torch.float8_e4m3fn, transpose_weight=True)
     with pytest.raises(RuntimeError, match="transpose_weight"):
         flux.GemmOnly(torch.int8, transpose_weight=True)
+
+
+def test_arrivals_at_another_cta_are_ordered_for_the_cluster():
+    """mbarrier.arrive defaults to the CTA's own scope; one whose target is another CTA's barrier (shared::cluster) must
+    say that it releases to the cluster. No other form of it is in the sources."""
+    import re
+
+    from flux_b200 import build
+
+    found = []
+    for f in sorted(build.CSRC.glob("*.cu*")):
+        found += re.findall(r"mbarrier\.arrive[.\w:]*shared::cluster[.\w:]*", f.read_text())
+    assert found == ["mbarrier.arrive.release.cluster.shared::cluster.b64"]
