@@ -267,21 +267,20 @@ inline void make_bands(GemmParams& p, int nseg, int tps, bool first_single, bool
 // Split-K tail: into how many parts along K each of the `tail_tiles` tiles of the last, partial wave of `workers`
 // workers is cut (1 = not at all). A part of fewer than 8 K blocks, or a cut that saves fewer than 32, costs more than
 // it gives: the parts exchange their accumulators in about 10 us, a K block takes 0.17 (narrow tiles) to 0.28 us.
-// Measured with a grid large enough to cut whole launches, uncut / cut: 256 x 512 x 512 12.6 / 15.6 us; 256 x 2048 x
-// 8192 54 / 29 us.
-// A reduce-scatter launch (`scatter`) keeps four K blocks per part and no minimum: its whole tiles end with peers'
-// partials to fetch, work that a cut spreads as well, and it has only been timed on several GPUs that way.
-__host__ __device__ __forceinline__ int splitk_parts(int tail_tiles, int workers, int num_kb, bool scatter) {
+// Launches of several ranks (`peers`) keep four K blocks per part and no minimum: they have only been timed on several
+// GPUs that way, where the tiles of the last wave also wait for peers' rows or end with peers' partials to fetch, work
+// that a cut spreads as well.
+__host__ __device__ __forceinline__ int splitk_parts(int tail_tiles, int workers, int num_kb, bool peers) {
   if (tail_tiles <= 0 || 2 * tail_tiles > workers) return 1;
-  const int by_workers = workers / tail_tiles, by_k = num_kb / (scatter ? 4 : 8);
+  const int by_workers = workers / tail_tiles, by_k = num_kb / (peers ? 4 : 8);
   const int sp = by_workers < 8 ? by_workers : 8;
   const int parts = sp < by_k ? sp : by_k;
-  return parts >= 2 && (scatter || num_kb - num_kb / parts >= 32) ? parts : 1;
+  return parts >= 2 && (peers || num_kb - num_kb / parts >= 32) ? parts : 1;
 }
 
 // The same for launch `p` of `total_tiles` tiles: the kernel's split, and the host's question whether it needs scratch.
 __host__ __device__ __forceinline__ int tail_split(const GemmParams& p, int total_tiles, int workers, int num_kb) {
-  return p.g_tiles == nullptr ? splitk_parts(total_tiles % workers, workers, num_kb, p.epi_mode == kEpiRsPush) : 1;
+  return p.g_tiles == nullptr ? splitk_parts(total_tiles % workers, workers, num_kb, p.epi_mode == kEpiRsPush || p.ag_flags != nullptr) : 1;
 }
 
 // Split-K tail: which part finishes the 32-column step `c` of a tail tile that is BN columns wide and cut into

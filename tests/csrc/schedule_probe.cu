@@ -112,3 +112,13 @@ extern "C" int probe_splitk_slots(const int* ops, int n, int* got, int* fresh) {
   }
   return kSplitkSlots;
 }
+
+// Parts of the last wave's tiles (tail_split of gemm_kernel.cuh): op 0 = one rank, 1 = all-gather, 2 = reduce-scatter.
+extern "C" int probe_tail_split(int op, int total_tiles, int workers, int num_kb) {
+  GemmParams p;
+  memset(&p, 0, sizeof(p));
+  int flag = 0;
+  p.epi_mode = op == 2 ? kEpiRsPush : kEpiStore;
+  if (op == 1) p.ag_flags = &flag;
+  return tail_split(p, total_tiles, workers, num_kb);
+}

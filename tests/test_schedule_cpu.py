@@ -46,6 +46,8 @@ def probe():
         fn.restype = C.c_int
     lib.probe_splitk_owner.argtypes = [C.c_int] * 4
     lib.probe_splitk_owners.argtypes = [C.c_int] * 3
+    lib.probe_tail_split.restype = C.c_int
+    lib.probe_tail_split.argtypes = [C.c_int] * 4
     lib.probe_splitk_slots.restype = C.c_int
     lib.probe_splitk_slots.argtypes = [C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.probe_rs_late_peers.restype = C.c_int
@@ -240,3 +242,18 @@ def test_split_scratch_is_never_shared_by_launches_that_may_overlap(probe):
     assert all(g == -1 for g in got[nslots:n]) and list(got[:n]) == list(got[n:2 * n]) and not any(fresh[nslots:2 * n])
     assert got[2 * n] == 2 and fresh[2 * n] == 1  # the slot that queue (5, 10) gave back
     assert got[2 * n + 1] == -1
+
+
+def test_where_the_last_wave_is_cut(probe):
+    """Both kinds of launches of several ranks cut a last wave that is at most half full into parts of at least four K
+    blocks; on one rank a part has at least eight, and the cut saves at least 32."""
+    rng = random.Random(5)
+    cases = [(rng.randint(1, 400), rng.choice([16, 37, 74, 148]), rng.randint(1, 200)) for _ in range(2000)]
+    for tiles, workers, num_kb in cases + [(8, 37, 16), (8, 37, 15), (75, 74, 40), (37 + 18, 37, 8)]:
+        tail = tiles % workers
+        most = min(8, workers // tail) if 0 < 2 * tail <= workers else 1
+        for op in (1, 2):
+            parts = min(most, num_kb // 4)
+            assert probe.probe_tail_split(op, tiles, workers, num_kb) == (parts if parts >= 2 else 1)
+        parts = min(most, num_kb // 8)
+        assert probe.probe_tail_split(0, tiles, workers, num_kb) == (parts if parts >= 2 and num_kb - num_kb // parts >= 32 else 1)
