@@ -229,6 +229,11 @@ def _make_moe_l1(group, max_tokens, hidden, nexperts, topk, dtype):
                                       input_dtype=dtype)
 
 
+def _is_stock_gather_rs(op) -> bool:
+    """Whether `op.forward_gather_rs` is the library's own: only then may a layer go around it to the same launches."""
+    return getattr(op.forward_gather_rs, "__func__", None) is _moe.GemmGroupedV3GatherRS.forward_gather_rs
+
+
 class MoEMLP(torch.nn.Module):
     """Tensor-parallel mixture-of-experts MLP (inference forward), tokens sharded in and out.
 
@@ -307,7 +312,7 @@ class MoEMLP(torch.nn.Module):
             gate, up = self._l0.forward_multiple_weights(x_shard.contiguous(), [self.w_gate, self.w_up], splits,
                                                          scatter_index)
             act = self.activation(gate) * up
-        if self.world == 1 and hasattr(self._l1, "_forward"):
+        if self.world == 1 and _is_stock_gather_rs(self._l1):
             # the counts stay on the device: reading them back would hold the host until layer 0 has run
             return self._l1._forward(act, self.w_down, None, splits, scatter_index.reshape(-1), output_vec_scale=row_scale)
         return self._l1.forward_gather_rs(act, self.w_down, splits.cpu(), scatter_index.reshape(-1),

@@ -233,6 +233,38 @@ def _moe_case(rank, world, gated=False):
     torch.testing.assert_close(y_shard, ref[rank * mpr:(rank + 1) * mpr], rtol=1e-4, atol=1e-5)
 
 
+def _moe_own_gather_rs_case(rank, world):
+    """A subclass of the op with a `forward_gather_rs` of its own is called through it."""
+    from flux_b200 import layers, moe
+    from oracle import golden
+
+    calls = []
+
+    class OwnL1(moe.GemmGroupedV3GatherRS):
+        def __init__(self, topk):
+            self._h = None
+            self.stand_in = FakeL1(None, topk)
+
+        def forward_gather_rs(self, *args, **kw):
+            calls.append(1)
+            return self.stand_in.forward_gather_rs(*args, **kw)
+
+    layers._scatter_index = lambda chosen, e: (golden.calc_scatter_index_stable(chosen), golden.calc_splits(chosen, e))
+    layers._make_moe_l0 = lambda group, *a: FakeL0(group)
+    layers._make_moe_l1 = lambda group, max_tokens, hidden, nexperts, topk, dtype: OwnL1(topk)
+    torch.manual_seed(5)
+    blk = layers.MoEMLP(16, 24, 4, 2, 6, None, dtype=torch.float32, device="cpu")
+    x = torch.randn(6, 16)
+    y = blk(x)
+    assert calls == [1]
+    blk._l1 = FakeL1(None, 2)
+    torch.testing.assert_close(y, blk(x), rtol=0, atol=0)
+
+
+def test_moe_block_own_gather_rs_world1():
+    run_distributed(_moe_own_gather_rs_case, 1, use_cuda=False)
+
+
 def test_moe_block_world2():
     run_distributed(_moe_case, 2, use_cuda=False)
 
