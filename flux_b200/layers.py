@@ -305,7 +305,7 @@ class MoEMLP(torch.nn.Module):
         chosen, weights = self.route(x_shard)
         scatter_index, splits = _scatter_index(chosen, self.nexperts)
         # routing weight of every expert-sorted row
-        row_scale = torch.empty_like(weights).view(-1).scatter_(0, scatter_index.view(-1).long(), weights.view(-1))
+        row_scale = weights.new_empty(weights.numel()).scatter_(0, scatter_index.reshape(-1).long(), weights.reshape(-1))
         if self.w_gate is None:
             act = self.activation(self._l0.forward(x_shard.contiguous(), self.w_up, splits, scatter_index))
         else:

@@ -265,6 +265,31 @@ def test_moe_block_own_gather_rs_world1():
     run_distributed(_moe_own_gather_rs_case, 1, use_cuda=False)
 
 
+def _moe_weights_layout_case(rank, world):
+    """`route` of a subclass may return its routing weights in any layout."""
+    from flux_b200 import layers
+    from oracle import golden
+
+    class ColumnMajorRouting(layers.MoEMLP):
+        def route(self, x_shard):
+            chosen, weights = super().route(x_shard)
+            return chosen, weights.t().contiguous().t()
+
+    layers._scatter_index = lambda chosen, e: (golden.calc_scatter_index_stable(chosen), golden.calc_splits(chosen, e))
+    layers._make_moe_l0 = lambda group, *a: FakeL0(group)
+    layers._make_moe_l1 = lambda group, max_tokens, hidden, nexperts, topk, dtype: FakeL1(group, topk)
+    torch.manual_seed(5)
+    blk = ColumnMajorRouting(16, 24, 4, 2, 6, None, dtype=torch.float32, device="cpu")
+    x = torch.randn(6, 16)
+    y = blk(x)
+    blk.__class__ = layers.MoEMLP
+    torch.testing.assert_close(y, blk(x), rtol=0, atol=0)
+
+
+def test_moe_block_weights_layout_world1():
+    run_distributed(_moe_weights_layout_case, 1, use_cuda=False)
+
+
 def test_moe_block_world2():
     run_distributed(_moe_case, 2, use_cuda=False)
 
