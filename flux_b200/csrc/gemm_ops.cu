@@ -482,7 +482,7 @@ static int launch_plain_inst(fluxb_comm* comm, PlainParams& p, uint32_t idesc, i
 // more (the partial last wave is cut along K) and no column padding to speak of. Measured back to back for 0.4 s
 // (us, 256 / 512 columns): 4096 x 49152 x 12288 3640 / 3490, 4096 x 12288 x 49152 3700 / 3540, 8192 x 8192 x 8192 811 / 785, fp8
 // 8192 x 8192 x 16384 812 / 791; with 64 K blocks fp8 8192 x 28672 x 8192 1408 / 1425, 2048 x 14336 x 4096 180 / 183.
-static bool wide_tile_wins(int sm_count, int m, int n, long long row_bytes) {
+bool wide_tile_wins(int sm_count, int m, int n, long long row_bytes) {
   const long long m_tiles = (m + 255) / 256, n_tiles = (n + 511) / 512;
   return (row_bytes + kRowBytes - 1) / kRowBytes >= 128 && m_tiles * n_tiles >= 3ll * (sm_count / 2) && n_tiles * 512ll * 64 <= n * 65ll;
 }

@@ -177,6 +177,9 @@ int encode_tmap_b16_store(CUtensorMap* out, const void* base, long long rows, lo
 int resolve_block_n(const fluxb_comm* comm, const GemmParams& p, const fluxb_tuning* tuning,
                     long long m_tiles_hint);
 
+// Whether a plain GEMM that gets 256 x 256 pair tiles takes 256 x 512 instead; `row_bytes` = bytes of K.
+bool wide_tile_wins(int sm_count, int m, int n, long long row_bytes);
+
 // Tiled-store map over a plain 16-bit output (see GemmParams::tmap_out); never fails, it only leaves the map invalid.
 void encode_out_map(GemmParams& p, void* out, long long rows, long long n, int out_type);
 

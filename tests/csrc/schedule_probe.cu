@@ -122,3 +122,5 @@ extern "C" int probe_tail_split(int op, int total_tiles, int workers, int num_kb
   if (op == 1) p.ag_flags = &flag;
   return tail_split(p, total_tiles, workers, num_kb);
 }
+
+extern "C" int probe_wide_tile(int sm_count, int m, int n, long long row_bytes) { return wide_tile_wins(sm_count, m, n, row_bytes) ? 1 : 0; }

@@ -58,18 +58,46 @@ def test_epilogue_edges(flux, m, n, k, tuning, bias, dtype):
     _check(flux, out, a, b, t)
 
 
+# (rows, columns, bytes of K) that get 256 x 512 tiles: 16 x 14 of them, three waves of 74 pairs and a cut rest
+WIDE_SHAPES = [(4000, 7160, 16384), (4096, 7168, 16384)]
+
+
+@pytest.fixture()
+def wide(flux):
+    """Asserts that the test's last launch had at most four work items a CTA: 256 x 256 tiles would have had seven."""
+    lib, comm = flux._lib.load(), flux.get_comm(None)
+    stamps = torch.zeros(torch.cuda.get_device_properties(0).multi_processor_count, 8, dtype=torch.int64, device="cuda")
+    flux._lib.check(lib.fluxb_comm_set_trace(comm.handle, stamps.data_ptr()))
+    yield
+    flux._lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
+    torch.cuda.synchronize()
+    assert 3 <= int(stamps[:, 7].max()) <= 4
+
+
 @pytest.mark.parametrize("kn", [False, True])
-@pytest.mark.parametrize("m,n,bias", [(4000, 7160, "row"), (4096, 7424, "full")])
-def test_wide_tiles(flux, m, n, bias, kn):
-    """128 K blocks and three waves of 256 x 512 tiles and a cut rest: rows and columns that end inside a tile."""
+@pytest.mark.parametrize("shape,bias", zip(WIDE_SHAPES, ("row", "full")))
+def test_wide_tiles(flux, wide, shape, bias, kn):
+    """Rows and columns that end inside a tile, and whole ones."""
+    m, n, _ = shape
     a, b, g = _inputs(m, n, 8192, BF16)
     t = torch.randn(1 if bias == "row" else m, n, generator=g, device="cuda").to(BF16)
     out = flux.GemmOnly(BF16, transpose_weight=kn).forward(a, b.t().contiguous() if kn else b, bias=t)
     _check(flux, out, a, b, t)
 
 
-def test_wide_tiles_int8(flux):
-    m, n, k = 4000, 7424, 16384
+@pytest.mark.parametrize("shape", WIDE_SHAPES)
+def test_wide_tiles_fp8(flux, wide, shape):
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(10)
+    a, b = (torch.randn(r, k, generator=g, device="cuda").to(torch.float8_e4m3fn) for r in (m, n))
+    sa, sb = (torch.rand(r, generator=g, device="cuda") * 0.01 + 0.001 for r in (m, n))
+    out = flux.GemmOnly(torch.float8_e4m3fn).forward(a, b, input_scale=sa, weight_scale=sb)
+    _check(flux, out, a.double() * sa[:, None].double(), b.double() * sb[:, None].double())
+
+
+@pytest.mark.parametrize("shape", WIDE_SHAPES)
+def test_wide_tiles_int8(flux, wide, shape):
+    m, n, k = shape
     g = torch.Generator(device="cuda").manual_seed(9)
     a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
     b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)

@@ -46,6 +46,8 @@ def probe():
         fn.restype = C.c_int
     lib.probe_splitk_owner.argtypes = [C.c_int] * 4
     lib.probe_splitk_owners.argtypes = [C.c_int] * 3
+    lib.probe_wide_tile.restype = C.c_int
+    lib.probe_wide_tile.argtypes = [C.c_int] * 3 + [C.c_longlong]
     lib.probe_tail_split.restype = C.c_int
     lib.probe_tail_split.argtypes = [C.c_int] * 4
     lib.probe_splitk_slots.restype = C.c_int
@@ -257,3 +259,16 @@ def test_where_the_last_wave_is_cut(probe):
             assert probe.probe_tail_split(op, tiles, workers, num_kb) == (parts if parts >= 2 else 1)
         parts = min(most, num_kb // 8)
         assert probe.probe_tail_split(0, tiles, workers, num_kb) == (parts if parts >= 2 and num_kb - num_kb // parts >= 32 else 1)
+
+
+def test_wide_tile_choice(probe):
+    """256 x 512 tiles from 128 K blocks and three waves on, without a sixty-fourth of column padding; the shapes that the
+    GPU tests of these tiles use are among them."""
+    from test_plain_gemm_gpu import WIDE_SHAPES
+
+    for m, n, row_bytes in WIDE_SHAPES:
+        assert probe.probe_wide_tile(148, m, n, row_bytes) == 1
+        assert resolve(probe, 1, m, n) == (256, 2)
+    assert probe.probe_wide_tile(148, 4096, 7168, 16383 - 127) == 0  # 127 K blocks
+    assert probe.probe_wide_tile(148, 3840, 7168, 16384) == 0  # 15 x 14 tiles: less than three waves
+    assert probe.probe_wide_tile(148, 4096, 7424, 16384) == 0  # the last of 15 column tiles is half empty
