@@ -384,6 +384,7 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
   p.timeout_ns = comm->timeout_ns;
   p.status = comm->status_dev;
   p.trace = comm->trace;
+  p.trace_ctas = comm->sm_count;
   int rc;
   if (p.w_kn) {
     FLUXB_REQUIRE(is_16bit(in_dtype), "a [K,N] weight needs 16-bit inputs (fp8 forbids transpose_weight)");

@@ -35,6 +35,7 @@ struct SkinnyParams {
   unsigned long long timeout_ns;
   int* status;
   unsigned long long* trace;
+  int trace_ctas;  // CTAs the timeline has room for: one per SM, of the up to two that this kernel runs there
 };
 
 template <int BN>
@@ -144,7 +145,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyParams p, const uint32_t idesc)
   const int kb0 = static_cast<int>(static_cast<long long>(part) * p.num_kb / split);
   const int kb1 = static_cast<int>(static_cast<long long>(part + 1) * p.num_kb / split);
   const int nkb = kb1 - kb0;
-  unsigned long long* tr = p.trace != nullptr && blockIdx.x < 148 ? p.trace + static_cast<size_t>(blockIdx.x) * 8 : nullptr;
+  unsigned long long* tr = p.trace != nullptr && static_cast<int>(blockIdx.x) < p.trace_ctas ? p.trace + static_cast<size_t>(blockIdx.x) * 8 : nullptr;
 
   auto load = [&](int i, int stage) {  // K block i of this part
     const uint32_t bar = bar_base + 8u * stage, dst = smem_base + stage * L::kStageBytes;

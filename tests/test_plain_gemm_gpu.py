@@ -75,7 +75,7 @@ def wide(flux):
 
 
 @pytest.mark.parametrize("kn", [False, True])
-@pytest.mark.parametrize("shape,bias", zip(WIDE_SHAPES, ("row", "full")))
+@pytest.mark.parametrize("shape,bias", list(zip(WIDE_SHAPES, ("row", "full"))))
 def test_wide_tiles(flux, wide, shape, bias, kn):
     """Rows and columns that end inside a tile, and whole ones."""
     m, n, _ = shape
@@ -290,3 +290,19 @@ def test_more_streams_than_scratch(flux):
             outs.append(call(a))
     comm.check_status()
     assert all(torch.equal(o, want) for o in outs)
+
+
+def test_timeline_has_room_for_one_cta_per_sm(flux):
+    """Few rows run up to two CTAs on an SM; the timeline buffer holds one per SM, and nothing is written behind it."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m, n, k = 16, 128 * sms, 1024  # one tile per SM, cut in two: twice as many CTAs as SMs
+    a, b, _ = _inputs(m, n, k, BF16)
+    lib, comm = flux._lib.load(), flux.get_comm(None)
+    stamps = torch.zeros(4 * sms, 8, dtype=torch.int64, device="cuda")
+    flux._lib.check(lib.fluxb_comm_set_trace(comm.handle, stamps.data_ptr()))
+    try:
+        out = flux.GemmOnly(BF16).forward(a, b)
+    finally:
+        flux._lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
+    _check(flux, out, a, b)
+    assert bool((stamps[:sms, 0] > 0).all()) and not bool(stamps[sms:].any())
