@@ -13,7 +13,7 @@ GemmRS.forward on its output. Global (M, N, K) are fixed, so N GPUs split the sa
 
 Prints ONE JSON line on rank 0. `value` = aggregate TFLOP/s over all GPUs with inputs resident in HBM;
 `e2e` = the same through host buffers (H2D of the activations and D2H of the result inside the timed
-region); `roofline` = the fused kernel against the measured bf16 tensor peak, with the NVLink side taken from
+region); `roofline` = the GEMM kernel against the measured bf16 tensor peak, with the NVLink side taken from
 the kernel's own timeline; `parity` = sampled fp64 dot products of both fused outputs, rows pushed by every
 peer included; `unfused` = cuBLAS + NCCL on the same box; `cpu_baseline` = the oracle on the host cores (a
 baseline, not the target); `fp8_ag_gemm` / `moe` = the two secondary configurations. A leg that fails records
@@ -95,6 +95,9 @@ def make_line(meas):
     use_burst = float(meas["timed_region_s"]) < 1.0
     peak = burst if use_burst else sustained
     nvl = meas.get("nvlink")
+    # dram__bytes_read.sum + dram__bytes_write.sum of a launch with M=4096, K=12288 and that many columns: on one rank the
+    # plain kernel with 256 x 512 tiles, on several the fused kernel
+    kernel, traffic, columns = ("plain_gemm_kernel", 643.5e6, 7168) if world == 1 else ("fused_gemm_kernel", 712.7e6, 6144)
     ag_link_s = ((world - 1) / world) * M * K0 * 2 / (NVLINK_GBS * 1e9)
     rs_link_s = ((world - 1) / world) * M * N1 * 2 / (NVLINK_GBS * 1e9)
     roofline = {
@@ -103,11 +106,10 @@ def make_line(meas):
                    else "of measured sustained peak (timed region >= 1 s)",
         "frac_of_burst_peak": ag_tflops / burst, "frac_of_sustained_peak": ag_tflops / sustained,
         "peak_burst": burst, "peak_sustained": sustained, "peak_source": f"{peak_src} cuBLAS bf16",
-        "kernel": "fused_gemm_kernel (AG-GEMM launch)",
-        # ncu (dram__bytes_read.sum + dram__bytes_write.sum) on the M=4096, N=6144, K=12288 launch: 712.7 MB;
-        # DRAM traffic grows with the number of 6144-column blocks a launch covers
-        "traffic": 712.7e6 * (N0 // world) / 6144.0,
-        "traffic_source": "ncu capture of the N=6144 launch (profiles/), scaled by N/6144",
+        "kernel": f"{kernel} (AG-GEMM launch)",
+        # DRAM traffic grows in proportion to the number of column blocks a launch covers
+        "traffic": traffic * (N0 // world) / columns,
+        "traffic_source": f"ncu capture of the N={columns} launch (profiles/), scaled by N/{columns}",
         "algorithmic_bytes": 2.0 * (M * K0 + (N0 // world) * K0 + M * (N0 // world)),
         "gemm_rs": {"achieved": rs_tflops, "frac": rs_tflops / peak},
         # the roofline time of a fused op is the slower of the tensor time and the NVLink time at 900 GB/s
@@ -827,7 +829,7 @@ def e2e_leg(ag, rs, a, b0, b1, c0, steps, world, barrier):
 # single-launch cases for profiler captures
 # ----------------------------------------------------------------------------------------------
 def run_kernel_only(args):
-    """Small single-GPU cases for profiler captures: the fused kernel alone at a per-rank shape of TP=8
+    """Small single-GPU cases for profiler captures: the op on one rank at a per-rank shape of TP=8
     (operands of a few hundred MB: larger than L2, far below the capture size limit).
       d0  : M=4096, N=6144,  K=12288 bf16 (AG-GEMM launch shape)
       d1  : M=4096, N=12288, K=6144  bf16 (GEMM-RS launch shape)

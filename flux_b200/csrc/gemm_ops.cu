@@ -26,7 +26,7 @@ static int take_splitk_slot(fluxb_comm* comm, Params& p, cudaStream_t stream) {
 
 template <int BN, int STAGES, int KIND, bool CTA2>
 static int launch_inst(fluxb_comm* comm, GemmParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
-  // (several ranks: the launch order of kernels that wait on one another stays the stream's)
+  // (several ranks: a kernel that waits for peers neither starts early nor lets the next one in early)
   const bool pdl = comm->world == 1;
   using L = SmemLayout<BN, STAGES, CTA2>;
   auto kern = fused_gemm_kernel<BN, STAGES, KIND, CTA2>;
@@ -84,7 +84,10 @@ static int pick_block_n(long long m_tiles, int n, int ctas, int per_cta_div, boo
   // cost = waves * tile width, with a small penalty for narrow tiles (more
   // operand traffic per flop); the candidate with the lowest cost wins.
   const int cand[4] = {256, 192, 128, 64};
-  const double pen[4] = {1.00, 1.15, 1.12, 1.30};  // measured: 192-wide tiles run ~12 % below 256-wide ones
+  // Time per output column against 256-wide pair tiles, K = 4096 (192 / 128 / 64 wide): one full wave 1.11 / 1.12 / 1.74, two
+  // 1.10 / 1.21 / 1.81, 8192 x 12288 (under the power cap) 1.26 / 1.33 / 2.16. The penalties are those of a wave or two, where
+  // the number of waves decides; that of 64 columns, mostly outputs too narrow for another width, is lower than measured.
+  const double pen[4] = {1.00, 1.15, 1.12, 1.30};
   int best = 256;
   double best_cost = 1e30;
   for (int i = 0; i < 4; ++i) {
@@ -348,11 +351,14 @@ static int skinny_split(int sm_count, int n_tiles, int num_kb, int bn) {
   return split;
 }
 
-// Where the skinny kernel takes over from the fused one's tiles (us, fused / skinny): every shape up to 64 rows
-// (16 x 4096 x 4096 22.8 / 9.0); above, shapes whose weights are too narrow to fill the GPU, so that K is cut at
-// least twice up to 128 rows (128 x 4096 x 4096 22.9 / 10.5 in four parts, but 128 x 14336 x 4096 26.4 / 30.9 in
-// one) and four times up to 256 (256 x 2048 x 8192 54 / 22.6, but 256 x 8192 x 8192 36 / 42 in two): the partial sums of
-// that many tokens take longer to exchange.
+// Where the skinny kernel takes over from tiles of 128 and more rows: every shape up to 64 rows; above, shapes whose
+// weights are too narrow to fill the GPU, so that K is cut at least twice up to 128 rows (128 x 14336 x 4096 takes 30.9 us in
+// one part, 25.9 in the plain kernel's tiles) and four times up to 256 (256 x 8192 x 8192 42 in two, 33.7 in tiles): the
+// partial sums of that many tokens take longer to exchange. Against the plain kernel (us, tiles / here): 16 x 4096 x 4096
+// 11.3 / 8.4, 48 x 6144 x 12288 35.7 / 30.3, 128 x 4096 x 4096 11.5 / 10.1, 256 x 4096 x 8192 21.6 / 20.3. The line was drawn
+// against the fused kernel's tiles, which are slower (256 x 2048 x 8192 54 us against the plain kernel's 17.8 and 18.5
+// here); with few K blocks the plain kernel is ahead on this side of it too: 64 x 8192 x 1024 5.5 / 7.6, 128 x 1024 x 512
+// 4.2 / 7.1, 200 x 2048 x 1024 5.5 / 10.3, 256 x 4096 x 4096 12.7 / 15.7.
 static bool skinny_wins(int sm_count, int m, int n, long long row_bytes) {
   if (m > kSkinnyMaxM) return false;
   if (m <= 64) return true;
@@ -645,7 +651,7 @@ int fluxb_gemm(fluxb_comm_t comm, const void* a, const void* b, void* c, int m, 
   const int eb = dtype_bytes(in_dtype);
   rc = out_type_of(out_dtype, &p.out_type);
   if (rc != FLUXB_OK) return rc;
-  // a caller who chose a tile shape or grid gets the fused kernel's
+  // a caller who chose a tile shape or grid gets those tiles, not the few-row kernel
   const bool chosen = tuning != nullptr && (tuning->block_n != 0 || tuning->cta_group != 0 || tuning->num_ctas != 0 || tuning->group_m != 0);
   if (!chosen && skinny_wins(comm->sm_count, m, n, static_cast<long long>(k) * eb) && comm->ranks_on_gpu <= 1 && p.out_type != kOutF32 &&
       ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(bias_mode != FLUXB_BIAS_NONE ? bias : nullptr)) & 3) == 0)

@@ -1,7 +1,9 @@
 // MoE grouped ops on top of the fused kernel's grouped mode.
 //
 // Layer 0 (all-gather + scatter + grouped GEMM) replaces
-// src/moe_ag_scatter/ths_op/gemm_grouped_v3_ag_scatter.cc:227-447: the token
+// src/moe_ag_scatter/ths_op/gemm_grouped_v3_ag_scatter.cc:227-447. On one rank a
+// table launch and the grouped GEMM, whose comm warps copy the caller's tokens
+// into expert order beside it, the first tiles' rows first. On several, the token
 // shard is pushed to every peer by the kernel's comm warps, the routing tables
 // (inverse permutation, per-expert M tiles, which source ranks a tile reads)
 // are built on the device - no device-to-host copy or host scheduling per call
@@ -11,7 +13,9 @@
 // room for that buffer and fetches A rows by token index with TMA gather4.)
 //
 // Layer 1 (grouped GEMM + top-k gather + reduce-scatter) replaces
-// src/moe_gather_rs/ths_op/gemm_grouped_v3_gather_rs.cc:595-820 in ONE launch,
+// src/moe_gather_rs/ths_op/gemm_grouped_v3_gather_rs.cc:595-820. On one rank:
+// a table launch, the grouped GEMM, and the top-k sum as a launch of its own
+// (moe_combine_kernel). On several, in ONE launch,
 // like the reference's threadblock-specialised kernel
 // (src/moe_gather_rs/sm90_gemm_array_threadblock_specialized.hpp:1315-1514):
 // the grouped GEMM writes a local [rows, N] buffer with the per-row /

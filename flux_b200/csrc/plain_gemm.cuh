@@ -49,7 +49,7 @@ struct PlainParams {
   const float* scale_b;
   uint16_t* out;
   const uint16_t* bias;
-  float* splitk_scratch;  // as in GemmParams; a part's slot is [quadrant][step][piece][lane]
+  float* splitk_scratch;  // as in GemmParams, null if nothing is cut; a part's slot is [quadrant][step][piece][lane]
   int* splitk_cnt;
   int* splitk_done;
   unsigned long long* trace;

@@ -243,7 +243,7 @@ class MoEMLP(torch.nn.Module):
       1. router: logits of this rank's tokens, top-k with softmax weights over the chosen experts; the choices
          and weights of all ranks are all-gathered (T x topk numbers) because the routing is global;
       2. `calc_scatter_index` gives each (token, k) pair its row in expert order;
-      3. layer 0: all-gather of the tokens + scatter + grouped GEMM in one kernel (`GemmGroupedV3AGScatter`);
+      3. layer 0: all-gather of the tokens + scatter + grouped GEMM (`GemmGroupedV3AGScatter`);
       4. activation; with `gated=True` (SwiGLU-style) a second up projection `w_gate` runs over the same gathered
          tokens (`forward_multiple_weights`: the all-gather happens once) and the activation is
          `act(gate) * up`;

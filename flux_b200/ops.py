@@ -358,7 +358,7 @@ class AGKernel:
 
     def gemm_only(self, input, weight, bias=None, output=None, input_scale=None, weight_scale=None,
                   output_scale=None, fast_accum=False, transpose_weight=False, tuning=None):
-        """Same kernel without communication: `input` is the full [M,K] matrix
+        """The GEMM without communication: `input` is the full [M,K] matrix
         (src/ag_gemm/ths_op/all_gather_gemm_op.cc:166-194)."""
         input, weight, output, bias_mode, m, n, k, flags = self._prep(
             input, weight, bias, output, input_scale, weight_scale, output_scale, transpose_weight, 1)
@@ -539,7 +539,7 @@ class GemmOnly:
     GEMM the reference uses as its unfused building block (src/pybind/gemm_only.cc; shapes and formulas in
     python/flux/cpp_mod.pyi:215-253): output = input[M,K] @ weight[N,K].T (weight [K,N] if transpose_weight),
     fp8 with scalar or per-row / per-channel scales, int8 (w8a8) with per-row x per-channel dequantisation, bias [M,N]
-    (16-bit) or [1,N]. Same kernel as the fused ops, without communication."""
+    (16-bit) or [1,N]. What the fused ops run on one rank."""
 
     def __init__(self, input_dtype, output_dtype=None, transpose_weight=False, use_fp8_gemm=False):
         if not (input_dtype in (torch.bfloat16, torch.float16) or _is_8bit(input_dtype)):
