@@ -26,7 +26,8 @@ static int take_splitk_slot(fluxb_comm* comm, Params& p, cudaStream_t stream) {
 
 template <int BN, int STAGES, int KIND, bool CTA2>
 static int launch_inst(fluxb_comm* comm, GemmParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
-  // (several ranks: a kernel that waits for peers neither starts early nor lets the next one in early)
+  // Several ranks: a kernel that waits for peers does not let the next one in early, and none starts early behind a library's
+  // collective, which may. CTAs that wait on this GPU would hold SMs of work that a peer waits for.
   const bool pdl = comm->world == 1;
   using L = SmemLayout<BN, STAGES, CTA2>;
   auto kern = fused_gemm_kernel<BN, STAGES, KIND, CTA2>;
@@ -307,7 +308,7 @@ int launch_fused_gemm(fluxb_comm* comm, GemmParams& p, int in_dtype,
 // few rows (skinny_gemm.cuh)
 // ---------------------------------------------------------------------------
 template <int BN, int KIND>
-static int launch_skinny_inst(const SkinnyParams& p, uint32_t idesc, int grid, cudaStream_t stream) {
+static int launch_skinny_inst(const SkinnyParams& p, uint32_t idesc, int grid, bool early, cudaStream_t stream) {
   auto kern = skinny_gemm_kernel<BN, KIND>;
   static bool configured[64] = {};
   int dev = 0;
@@ -331,7 +332,7 @@ static int launch_skinny_inst(const SkinnyParams& p, uint32_t idesc, int grid, c
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = early ? 2 : 1;
   FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, idesc));
   return FLUXB_OK;
 }
@@ -409,10 +410,11 @@ static int launch_skinny(const fluxb_comm* comm, const void* a, const void* b, v
   p.split = skinny_split(comm->sm_count, n_tiles, p.num_kb, bn);
   const int grid = n_tiles * p.split;
   const int kind = kind_of(in_dtype);
+  const bool early = comm->world == 1;  // (see launch_inst)
 #define FLUXB_SKINNY(BN_)                                                    \
-  (kind == 0 ? launch_skinny_inst<BN_, 0>(p, idesc, grid, stream)            \
-   : kind == 1 ? launch_skinny_inst<BN_, 1>(p, idesc, grid, stream)          \
-               : launch_skinny_inst<BN_, 2>(p, idesc, grid, stream))
+  (kind == 0 ? launch_skinny_inst<BN_, 0>(p, idesc, grid, early, stream)            \
+   : kind == 1 ? launch_skinny_inst<BN_, 1>(p, idesc, grid, early, stream)          \
+               : launch_skinny_inst<BN_, 2>(p, idesc, grid, early, stream))
   switch (bn) {
     case 16: return FLUXB_SKINNY(16);
     case 32: return FLUXB_SKINNY(32);
@@ -479,7 +481,7 @@ static int launch_plain_inst(fluxb_comm* comm, PlainParams& p, uint32_t idesc, i
   }
   p.split_div.set(static_cast<uint32_t>(p.split));
   cfg.gridDim = dim3(workers * per, 1, 1);
-  cfg.numAttrs = 2;
+  cfg.numAttrs = comm->world == 1 ? 2 : 1;  // (see launch_inst)
   FLUXB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, idesc));
   return FLUXB_OK;
 }

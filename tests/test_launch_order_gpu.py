@@ -86,3 +86,33 @@ def test_nothing_starts_beside_a_launch_that_waits_for_a_peer(flux):
     finally:
         _lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
         rk.close()
+
+
+@pytest.mark.parametrize("m", [16, 512])  # few rows, plain
+def test_with_several_ranks_no_gemm_starts_early(flux, m):
+    """Behind a launch that lets the next one in early (one CTA, several ms), a GEMM of a rank of two waits outside."""
+    from flux_b200 import _lib
+
+    lib, n, k = _lib.load(), 256, 512
+    a, b = torch.ones(m, k, device="cuda", dtype=BF16), torch.ones(n, k, device="cuda", dtype=BF16)
+    out = torch.empty(m, n, device="cuda", dtype=BF16)
+    big = torch.zeros(2048, 8192, device="cuda", dtype=BF16)
+    comm = flux.get_comm(None)
+    words = torch.cuda.get_device_properties(0).multi_processor_count * 8
+    first, second = (torch.zeros(words, dtype=torch.int64, device="cuda") for _ in range(2))
+    two = C.c_void_p()
+    _lib.check(lib.fluxb_comm_create(0, 2, C.byref(two)))
+    try:
+        _lib.check(lib.fluxb_comm_set_trace(comm.handle, _p(first)))
+        _lib.check(lib.fluxb_comm_set_trace(two, _p(second)))
+        for _ in range(2):  # the first round loads the kernels
+            flux.GemmOnly(BF16).forward(big, big, tuning={"block_n": 256, "cta_group": 1, "num_ctas": 1})
+            _lib.check(lib.fluxb_gemm(two, _p(a), _p(b), _p(out), m, n, k, _lib.BF16, _lib.BF16, None, 0, None, None, 1.0, 0, None,
+                                      _stream()))
+            torch.cuda.synchronize()
+        assert bool((out == k).all())
+        entered = second.view(-1, 8)[:, 0]
+        assert int(entered[entered > 0].min()) >= int(first.view(-1, 8)[0, 3])
+    finally:
+        _lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
+        lib.fluxb_comm_destroy(two)
