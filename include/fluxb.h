@@ -132,7 +132,7 @@ int fluxb_run_ranks(fluxb_comm_t const* comms, int nranks, fluxb_stream_t stream
  * The TP=1 degenerate of both fused ops; also what AGKernel.gemm_only runs
  * (src/ag_gemm/ths_op/all_gather_gemm_op.cc:166-194). A and B are row-major
  * with K contiguous. scale_a / scale_b may be NULL. Calls on several streams and in captured graphs may run side by
- * side; of the executables made from one graph, only one at a time. A communicator keeps
+ * side, but no graph beside a copy of itself (a second executable, a child graph). A communicator keeps
  * scratch for the cut last waves of eight streams or graphs; on any further ones large launches run uncut: slower
  * (by up to a wave of tiles), and with the sums of those tiles in another order. */
 int fluxb_gemm(fluxb_comm_t comm, const void* a, const void* b, void* c, int m, int n, int k,

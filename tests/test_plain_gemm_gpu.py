@@ -262,6 +262,22 @@ def test_cut_launches_in_graphs_beside_eager_ones(flux):
     assert torch.equal(outs[0], want) and torch.equal(outs[1], want2) and torch.equal(outs[2], want)
 
 
+def test_eager_cut_launch_while_another_stream_captures(flux):
+    """The stream that a launch goes to is asked for its identity without disturbing a capture on another one."""
+    comm, a, a2, call = _cut_launch(flux, BF16, 74)
+    want, want2 = call(a), call(a2)
+    outs = [torch.empty_like(want) for _ in range(2)]
+    eager, stream, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    comm.check_status()
+    with torch.cuda.graph(graph, stream=stream):
+        call(a, outs[0])
+        with torch.cuda.stream(eager):
+            call(a2, outs[1])
+    graph.replay()
+    comm.check_status()
+    assert torch.equal(outs[0], want) and torch.equal(outs[1], want2)
+
+
 def test_graphs_give_their_scratch_back(flux):
     """More graphs, one after the other, than there is scratch for: the last is cut like the first (the same sums)."""
     comm, a, _, call = _cut_launch(flux, BF16, 74)
