@@ -685,6 +685,7 @@ int fluxb_gemm(fluxb_comm_t comm, const void* a, const void* b, void* c, int m, 
       bn = 512;
     return launch_plain(comm, p, a, b, in_dtype, bn, cg, tuning, static_cast<cudaStream_t>(stream));
   }
+  FLUXB_REQUIRE_ALIGNED(c, "gemm: the output");
   rc = encode_tmap_2d(&p.tmap_a, a, in_dtype, m, k, static_cast<long long>(k) * eb, kBM);
   if (rc != FLUXB_OK) return rc;
   encode_out_map(p, c, m, n, p.out_type);
@@ -781,6 +782,7 @@ int fluxb_ag_gemm_forward(fluxb_ag_gemm_t op, const void* a_shard, int m_local, 
   FLUXB_REQUIRE(bias_mode == FLUXB_BIAS_NONE || bias != nullptr, "ag_gemm_forward: bias is NULL");
   FLUXB_REQUIRE(scale_a_shard == nullptr || op->has_scales,
                 "ag_gemm_forward: per-row input scales need scale buffers at create time");
+  if (world > 1) FLUXB_REQUIRE_ALIGNED(c, "ag_gemm_forward: the output");
   const int eb = dtype_bytes(op->in_dtype);
   const long long row_bytes = static_cast<long long>(k) * eb;
 
@@ -969,6 +971,7 @@ int fluxb_gemm_rs_forward(fluxb_gemm_rs_t op, const void* a, const void* b, int 
                       scale_a, scale_b, alpha, flags, tuning, stream_);
   FLUXB_REQUIRE(bias_mode == FLUXB_BIAS_NONE || op->out_dtype == FLUXB_BF16,
                 "gemm_rs_forward: bias needs a bf16 output");
+  FLUXB_REQUIRE_ALIGNED(out, "gemm_rs_forward: the output");
   // w8a8: the bias is applied by rank 0 only (src/gemm_rs/ths_op/gemm_reduce_scatter.cc:596-599)
   if (is_int8(op->in_dtype) && comm->rank != 0) bias_mode = FLUXB_BIAS_NONE;
 

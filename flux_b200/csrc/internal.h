@@ -39,6 +39,10 @@ void set_error(const char* fmt, ...);
                  __FILE__, __LINE__);                                                 \
   } while (0)
 
+// Rows of a buffer that kernels read or write 16 bytes at a time with plain vector accesses (tensor maps check theirs).
+#define FLUXB_REQUIRE_ALIGNED(ptr, what) \
+  FLUXB_REQUIRE((reinterpret_cast<uintptr_t>(ptr) & 15) == 0, what " must be 16-byte aligned")
+
 // Launches with the programmatic-dependent-launch attribute: the kernel must call pdl_wait() before it touches global
 // memory, and pdl_trigger() for the next one to be let in early.
 template <class... P, class... A>

@@ -486,6 +486,8 @@ int fluxb_moe_ag_scatter_forward(fluxb_moe_ag_scatter_t op, const void* tokens_s
   FLUXB_REQUIRE(ntokens_local >= 1 && ntokens <= op->max_ntokens,
                 "moe_ag_scatter_forward: ntokens_local=%d * world=%d exceeds max_ntokens=%d", ntokens_local, world, op->max_ntokens);
   const bool reuse = tokens_shard == nullptr;
+  FLUXB_REQUIRE_ALIGNED(tokens_shard, "moe_ag_scatter_forward: the tokens");
+  FLUXB_REQUIRE_ALIGNED(out, "moe_ag_scatter_forward: the output");
   FLUXB_REQUIRE(!reuse || (op->last_parity >= 0 && op->last_ntokens == ntokens_local),
                 "moe_ag_scatter_forward: no gathered tokens of this size to reuse");
   const int eb = dtype_bytes(op->in_dtype);
@@ -766,6 +768,7 @@ static int gather_rs_forward(fluxb_moe_gather_rs* op, const void* x, int m, int 
                              fluxb_stream_t stream_) {
   FLUXB_REQUIRE(op != nullptr && x != nullptr && weights != nullptr && routing_idx_dev != nullptr && out != nullptr,
                 "moe_gather_rs_forward: NULL argument");
+  FLUXB_REQUIRE_ALIGNED(out, "moe_gather_rs_forward: the output");
   fluxb_comm* comm = op->comm;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int world = comm->world;
@@ -968,6 +971,7 @@ extern "C" int fluxb_moe_scatter_gemm_static(fluxb_comm_t comm, const void* toke
                                              const fluxb_tuning* tuning, fluxb_stream_t stream_) {
   FLUXB_REQUIRE(comm != nullptr && tokens != nullptr && weights != nullptr && splits_dev != nullptr &&
                     scatter_index_dev != nullptr && out != nullptr, "moe_scatter_gemm_static: NULL argument");
+  FLUXB_REQUIRE_ALIGNED(out, "moe_scatter_gemm_static: the output");
   FLUXB_REQUIRE(comm->world == 1, "moe_scatter_gemm_static: needs a world-1 communicator (got world=%d)", comm->world);
   FLUXB_REQUIRE(is_16bit(in_dtype) || is_fp8(in_dtype), "moe_scatter_gemm_static: input dtype %d unsupported", in_dtype);
   FLUXB_REQUIRE(out_dtype == FLUXB_BF16 || out_dtype == FLUXB_F16, "moe_scatter_gemm_static: output dtype %d unsupported", out_dtype);

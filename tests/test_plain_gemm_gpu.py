@@ -322,3 +322,27 @@ def test_timeline_has_room_for_one_cta_per_sm(flux):
         flux._lib.check(lib.fluxb_comm_set_trace(comm.handle, None))
     _check(flux, out, a, b)
     assert bool((stamps[:sms, 0] > 0).all()) and not bool(stamps[sms:].any())
+
+
+def test_misaligned_vectors_are_refused(flux):
+    """The kernels move output rows and MoE tokens 16 bytes at a time: anything else is an error of the call, unless the few-row
+    kernel (4 bytes) takes it."""
+    m, n, k = 300, 64, 128
+    a, b, g = _inputs(m, n, k, BF16)
+    shifted = lambda rows, cols, by: torch.zeros(rows * cols + by, dtype=BF16, device="cuda")[by:].view(rows, cols)
+    op = flux.GemmOnly(BF16)
+    for by in (1, 2, 4):
+        with pytest.raises(RuntimeError, match="aligned"):
+            op.forward(a, b, output_buf=shifted(m, n, by))
+    with pytest.raises(RuntimeError, match="aligned"):
+        op.forward(a[:16], b, output_buf=shifted(16, n, 1))
+    out = op.forward(a[:16], b, output_buf=shifted(16, n, 2))
+    _check(flux, out, a[:16], b)
+    tokens, experts, topk = 8, 2, 2
+    si, splits = flux.calc_scatter_index(torch.tensor([[0, 1]] * tokens, dtype=torch.int32, device="cuda"), torch.empty(2), return_splits=True)
+    l0 = flux.GemmGroupedV3AGScatter(flux.DistEnvTPWithEP(None, 1, None), flux.MoeArguments(tokens, k, n, experts, topk, BF16))
+    w = torch.zeros(experts, n, k, dtype=BF16, device="cuda")
+    with pytest.raises(RuntimeError, match="tokens must be 16-byte aligned"):
+        l0.forward(shifted(tokens, k, 1), w, splits, si)
+    with pytest.raises(RuntimeError, match="output must be 16-byte aligned"):
+        l0.forward(a[:tokens], w, splits, si, outputs_buf=shifted(tokens * topk, n, 1))
