@@ -215,7 +215,8 @@ int resolve_block_n(const fluxb_comm* comm, const GemmParams& p, const fluxb_tun
     if (m_tiles <= 0) m_tiles = static_cast<long long>(p.nseg) * ((p.seg_rows + tile_m - 1) / tile_m);
     int share = comm->ranks_on_gpu > 1 ? ((comm->sm_count / comm->ranks_on_gpu) & ~1) : comm->sm_count;
     int ctas = (tuning != nullptr && tuning->num_ctas > 0 && tuning->num_ctas < share) ? tuning->num_ctas : share;
-    bn = pick_block_n(m_tiles, p.N, cg == 2 ? ctas / 2 : ctas, cg == 2 ? 2 : 1, p.b_mn_major != 0);
+    const int workers = cg == 2 ? ctas / 2 : ctas;  // (one CTA of a caller's choice still makes one pair)
+    bn = pick_block_n(m_tiles, p.N, workers > 0 ? workers : 1, cg == 2 ? 2 : 1, p.b_mn_major != 0);
   }
   return bn;
 }

@@ -162,6 +162,8 @@ def test_tile_shape_choice(probe):
     # the caller's tuning wins
     assert resolve(probe, 8, 512, 6144, bn=128, cg=1) == (128, 1)
     assert resolve(probe, 8, 512, 6144, cg=1)[1] == 1
+    # one CTA, and pairs: the width is chosen for one pair
+    assert resolve(probe, 1, 4096, 6144, cg=2, ctas=1) == resolve(probe, 1, 4096, 6144, cg=2, ctas=2)
 
 
 def _band_segments(segs, nseg):
