@@ -873,7 +873,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       for (; ok && get_item(it, t, kb0, kb1, part); ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget))
+        if (!mbar_wait<CTA2>(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget))
           break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);

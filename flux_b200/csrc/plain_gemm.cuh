@@ -231,7 +231,7 @@ plain_gemm_kernel(const __grid_constant__ PlainParams p, const uint32_t idesc) {
       for (; ok && get_item(it, t, kb0, kb1, part); ++it) {
         const int acc = ACCS == 2 ? it & 1 : 0;
         const uint32_t acc_phase = (ACCS == 2 ? it >> 1 : it) & 1;
-        if (!mbar_wait(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget)) break;
+        if (!mbar_wait<CTA2>(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = kb0; kb < kb1; ++kb) {

@@ -77,6 +77,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// The other end of mbar_arrive_cluster: this CTA's barrier, arrivals from the whole cluster.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 P, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(20000u)
+      : "memory");
+  return ok != 0;
+}
 
 // The abort word of a CTA: non-zero means some role has given up, and every other role must leave
 // its loop too. In a CTA pair the word of the partner CTA is raised as well (a store through
@@ -99,12 +111,15 @@ __device__ __forceinline__ bool abort_seen(const AbortWord& ab) {
 // Bounded mbarrier wait.
 // `backoff_ns` > 0 sleeps between polls: for waits that normally last many microseconds (an
 // accumulator that is still being computed), so that idle warps do not burn issue slots and power.
+// CLUSTER: for arrivals by mbar_arrive_cluster.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const AbortWord& ab,
                                           int code, uint64_t budget_ns, uint32_t backoff_ns = 0) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto done = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+  if (done()) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t n = 0;
-  while (!mbar_try_wait(bar, parity)) {
+  while (!done()) {
     if (backoff_ns != 0) __nanosleep(backoff_ns);
     if ((++n & 31u) == 0u) {
       if (abort_seen(ab)) return false;
@@ -372,10 +387,13 @@ __device__ __forceinline__ uint2 ld_shared_cluster_v2(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(cluster_addr) : "memory");
   return v;
 }
-// Arrival at a barrier of another CTA of the cluster. The default scope is the CTA, which does not order the arriving
-// warps' reads of tensor memory before what the other CTA issues once it has seen them.
+// Arrival at a barrier of another CTA of the cluster, which announces that this warp's reads of tensor memory are done. The
+// default scope is the CTA: it would not order them before what the other CTA issues. Both ends have the cluster's, and
+// tcgen05.wait::ld and tcgen05.fence::before_thread_sync here, ::after_thread_sync there, order the tensor memory accesses
+// around them. Relaxed, because nothing in ordinary memory is handed over: a release would wait for all of the warp's
+// earlier stores at every tile (fp8 8192 x 7168 x 8192 386 us against 383, MLP of 4096 x 12288 x 49152 7266 / 7170).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_2cta(uint32_t smem_dst, uint32_t ncols) {

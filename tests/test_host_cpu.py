@@ -105,8 +105,8 @@ def test_gemm_only_rejects_unsupported_modes():
 
 
 def test_arrivals_at_another_cta_are_ordered_for_the_cluster():
-    """mbarrier.arrive defaults to the CTA's own scope; one whose target is another CTA's barrier (shared::cluster) must
-    say that it releases to the cluster. No other form of it is in the sources."""
+    """mbarrier.arrive and try_wait default to the CTA's own scope; an arrival whose target is another CTA's barrier
+    (shared::cluster) and the wait for it must name the cluster's. No other form of it is in the sources."""
     import re
 
     from flux_b200 import build
@@ -114,4 +114,5 @@ def test_arrivals_at_another_cta_are_ordered_for_the_cluster():
     found = []
     for f in sorted(build.CSRC.glob("*.cu*")):
         found += re.findall(r"mbarrier\.arrive[.\w:]*shared::cluster[.\w:]*", f.read_text())
-    assert found == ["mbarrier.arrive.release.cluster.shared::cluster.b64"]
+    assert found == ["mbarrier.arrive.relaxed.cluster.shared::cluster.b64"]
+    assert "mbarrier.try_wait.parity.relaxed.cluster" in (build.CSRC / "ptx.cuh").read_text()
