@@ -446,6 +446,9 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint64_t budget = p.timeout_ns;
+  // Waits inside the CTA (and for the other parts of a cut tile) that may follow from a wait for a peer last an eighth longer:
+  // the peer's wait is the one to expire, and its code the one to be reported.
+  const uint64_t budget_in = budget + (budget >> 3);
   const int half = CTA2 ? static_cast<int>(cluster_ctarank()) : 0;  // rank inside the CTA pair
   const bool leader = half == 0;
   const int tile_first = CTA2 ? (cta_id >> 1) : cta_id;
@@ -703,7 +706,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       const int i2 = gi[r0 + 2 < nr ? r0 + 2 : 0];
       const int i3 = gi[r0 + 3 < nr ? r0 + 3 : 0];
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(bar_empty(stage), phase ^ 1u, ab, kStatusTimeoutSmemEmpty, budget, 40)) {
+        if (!mbar_wait(bar_empty(stage), phase ^ 1u, ab, kStatusTimeoutSmemEmpty, budget_in, 40)) {
           ok = false;
           break;
         }
@@ -825,7 +828,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
             if (!ok) break;
             fence_proxy_async();
           }
-          if (!mbar_wait(bar_empty(stage), phase ^ 1u, ab, kStatusTimeoutSmemEmpty, budget, 40)) {
+          if (!mbar_wait(bar_empty(stage), phase ^ 1u, ab, kStatusTimeoutSmemEmpty, budget_in, 40)) {
             ok = false;
             break;
           }
@@ -873,12 +876,12 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       for (; ok && get_item(it, t, kb0, kb1, part); ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait<CTA2>(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget))
+        if (!mbar_wait<CTA2>(bar_tempty(acc), acc_phase ^ 1u, ab, kStatusTimeoutTmemEmpty, budget_in))
           break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_full(stage), phase, ab, kStatusTimeoutSmemFull, budget)) {
+          if (!mbar_wait(bar_full(stage), phase, ab, kStatusTimeoutSmemFull, budget_in)) {
             ok = false;
             break;
           }
@@ -945,7 +948,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
       TileCoord tc;
       decode_tile<BN, TILE_M>(p, t, m_tiles, n_tiles, tps, half, tc);
       // (one verdict for the whole warp: what follows are warp-wide operations)
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull(acc), acc_phase, ab, kStatusTimeoutTmemFull, budget, 300))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull(acc), acc_phase, ab, kStatusTimeoutTmemFull, budget_in, 300))) break;
       tc_fence_after();
       // split-K tail: where this warp's 32 rows of a tail tile's partial accumulators live. Inside a part's slot the
       // four columns q of 32-column step c of lane l are 16-byte piece (c * 8 + q) * 32 + l, so that every access of
@@ -989,7 +992,7 @@ __device__ __forceinline__ void fused_gemm_body(const GemmParams& p, const uint3
         int okw = 1;
         if (lane == 0) {
           red_add_release_sys(sk_cnt, 1);
-          if (part < sk_owners) okw = flag_wait_eq(sk_cnt, split, ab, kStatusTimeoutTmemFull, budget) ? 1 : 0;
+          if (part < sk_owners) okw = flag_wait_eq(sk_cnt, split, ab, kStatusTimeoutTmemFull, budget_in) ? 1 : 0;
           // the last part through clears both counters for the next launch
           if (okw && atomicAdd(sk_done, 1) == split - 1) {
             *sk_cnt = 0;

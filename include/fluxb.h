@@ -93,6 +93,8 @@ int fluxb_device_supported(void);
  * process group, as Group::all_gather_cpu does, flux_shm.cc:161-168). */
 int fluxb_comm_create(int rank, int world, fluxb_comm_t* out);
 int fluxb_comm_destroy(fluxb_comm_t comm);
+/* Longest wait for a peer (default 10 s); waits inside a kernel that may follow from one last an eighth longer, so that the
+ * status word names the peer's. */
 int fluxb_comm_set_timeout_ms(fluxb_comm_t comm, int timeout_ms);
 /* Optional timeline of the fused kernel (the reference has only host-side profiling,
  * python/flux/util.py:111-172): device_buffer = 8 x uint64 per CTA (64 B x SM count), filled by every
